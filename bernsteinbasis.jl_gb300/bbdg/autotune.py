@@ -5,7 +5,7 @@ block; every degree-specialised FP32 variant of its physics and degree in the li
 registry, and the generic kernel's tiles) over a few LSRK steps on the solver's own mesh with
 CUDA events, keeps the fastest, and caches the choice per (physics, N, dtype, element count,
 device name, library content hash) in a JSON file next to the built library (the element
-count decides which tiles divide the mesh; a rebuilt library invalidates the entries). The
+count decides how many tiles each block gets; a rebuilt library invalidates the entries). The
 field vector width is not a tuning dimension: it is fixed by the physics in the specialised
 kernels (wave: one 16-byte w entry per point; Maxwell: three 8-byte pieces).
 """
@@ -71,12 +71,12 @@ def _load():
 
 
 def candidates(solver):
-    """Every compiled specialised variant for the solver's (physics, N) whose tile divides
-    its element count (FP32 only), then the generic tiles; each is timed, the fastest kept."""
+    """Every compiled specialised variant for the solver's (physics, N) (FP32 only; a last
+    tile may be partial), then the generic tiles; each is timed, the fastest kept."""
     spec = []
     if solver.dtype == torch.float32:
         spec = [("specialised", epb, nt) for (N, phys, epb, nt) in compiled_variants()
-                if N == solver.N and phys == solver.physics and solver.K % epb == 0]
+                if N == solver.N and phys == solver.physics]
     return spec + GENERIC
 
 

@@ -163,7 +163,7 @@ int build_desc(bb_batch* b) {
   for (int p = 0; p < np; ++p) {
     const bb_batch_problem& pr = b->probs[p];
     if (sizeof(T) == 4 && a16(pr.q) && a16(pr.res) && a16(pr.geo) && a16(pr.conn)) {
-      const int idx = bb_fast_find(pr.N, pr.physics, 0, 0, pr.K);
+      const int idx = bb_fast_find(pr.N, pr.physics, 0, 0);
       int e = 0, th = 0;
       size_t sm = 0;
       if (idx >= 0 && bb_fast_variant_info(idx, &e, &th, &sm) == BB_OK && sm <= ctx->smem_optin)

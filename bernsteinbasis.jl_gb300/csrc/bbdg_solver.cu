@@ -386,7 +386,7 @@ extern "C" int bb_solver_create(bb_ctx* ctx, int physics, int N, int64_t K, int 
     s->smem = sm;
   }
   if (dtype == BB_F32) {
-    const int idx = bb_fast_find(N, physics, 0, 0, K);
+    const int idx = bb_fast_find(N, physics, 0, 0);
     int e = 0, th = 0;
     size_t sm = 0;
     if (idx >= 0 && bb_fast_variant_info(idx, &e, &th, &sm) == BB_OK && sm <= ctx->smem_optin) {
@@ -437,7 +437,7 @@ extern "C" int bb_solver_set_tile(bb_solver* s, int epb, int threads) {
   if (!s) return BB_ERR_ARG;
   // degree-specialised FP32 variants first, unless the generic kernel was requested
   if (s->dtype == BB_F32 && !s->generic_only) {
-    const int idx = bb_fast_find(s->N, s->physics, epb, threads, s->K);
+    const int idx = bb_fast_find(s->N, s->physics, epb, threads);
     int e = 0, th = 0;
     size_t sm = 0;
     if (idx >= 0 && bb_fast_variant_info(idx, &e, &th, &sm) == BB_OK && sm <= s->ctx->smem_optin) {
@@ -469,7 +469,7 @@ extern "C" int bb_solver_set_kernel(bb_solver* s, int kind) {
   if (kind != 0 && kind != 1) return bb_fail(s->ctx, BB_ERR_ARG, "kind must be 0 or 1");
   s->generic_only = kind;
   if (kind == 1 && s->fast >= 0) return bb_solver_set_tile(s, s->epb, kThreads);
-  if (kind == 0 && s->fast < 0 && s->dtype == BB_F32 && bb_fast_find(s->N, s->physics, 0, 0, s->K) >= 0)
+  if (kind == 0 && s->fast < 0 && s->dtype == BB_F32 && bb_fast_find(s->N, s->physics, 0, 0) >= 0)
     return bb_solver_set_tile(s, 0, 0);
   return BB_OK;
 }

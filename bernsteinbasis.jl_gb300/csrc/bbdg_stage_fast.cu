@@ -10,12 +10,11 @@ BB_FAST_VARIANTS(BB_EXTERN)
 #undef BB_EXTERN
 
 // The public tile description is (elements per block, threads per block).
-int bb_fast_find(int N, int physics, int epb, int threads, int64_t K) {
+int bb_fast_find(int N, int physics, int epb, int threads) {
   int idx = 0;
 #define BB_FIND(n_, p_, e_, t_)                                                        \
   if (N == n_ && physics == p_ && (epb == 0 || epb == e_) &&                           \
-      (threads == 0 || threads == FastLayout<n_, p_, e_, t_>::NT) &&                   \
-      (K <= 0 || K % e_ == 0))                                                         \
+      (threads == 0 || threads == FastLayout<n_, p_, e_, t_>::NT))                     \
     return idx;                                                                        \
   ++idx;
   BB_FAST_VARIANTS(BB_FIND)

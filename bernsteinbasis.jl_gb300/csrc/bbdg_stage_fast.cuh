@@ -20,6 +20,7 @@ struct FastStageParams {
   int* status;
   uint32_t wait_iters;   // polls of a bounded mbarrier wait before it gives up (0 = 2^24)
   int fault;             // test only: 1 = one bulk copy is left out (a wait then runs out)
+  int vec;               // floats per copy the field rows are aligned for: 4 = bulk copies, 2, 1
   // volume phase: warp-round g = r * (TPE / 32) + warp forms w(beta) for beta = vstart[g] +
   // lane, lane < vlen[g] (filled by the launcher)
   uint16_t vstart[16];
@@ -33,8 +34,8 @@ struct FastLaunch {
   int fault;            // copied into FastStageParams (the context's test-only fault mode)
 };
 
-// Index of the compiled variant for (N, physics, elements per block, threads), 0 = any,
-// usable for K elements (K must be a multiple of the tile; K <= 0: any); -1 if none.
-int bb_fast_find(int N, int physics, int epb, int threads, int64_t K);
+// Index of the compiled variant for (N, physics, elements per block, threads), 0 = any; -1 if
+// none. Any element count will do: the last tile may be partial.
+int bb_fast_find(int N, int physics, int epb, int threads);
 int bb_fast_variant_info(int idx, int* epb, int* threads, size_t* smem);
 int bb_fast_launch(int idx, const FastLaunch& fl, const FastStageParams& P, cudaStream_t st);

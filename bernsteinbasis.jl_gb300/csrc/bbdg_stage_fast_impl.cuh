@@ -87,9 +87,10 @@ struct FastLayout {
   static constexpr int QBYTES = NF * EPB * NP * 4;            // q tile, [NF][EPB][NP]
   static constexpr int GEOBYTES = EPB * BB_GEO_STRIDE * 4;     // [EPB][24]
   static constexpr int CONNBYTES = EPB * 16;                   // [EPB][4] int32
-  static constexpr int SLOT = ((QBYTES + GEOBYTES + CONNBYTES) + 15) / 16 * 16;
+  static constexpr int GEO_O = (QBYTES + 15) / 16 * 16;        // geometry within a slot
+  static constexpr int SLOT = GEO_O + GEOBYTES + CONNBYTES;
   static constexpr int RES_B = 2 * SLOT;                       // after the two q slots
-  static constexpr int G_B = RES_B + QBYTES;                   // [EPB*4][NPS][NCH] face stacks
+  static constexpr int G_B = RES_B + GEO_O;                    // [EPB*4][NPS][NCH] face stacks
   static constexpr int X_B = G_B + (NCHAIN * NPS * 4 + 15) / 16 * 16;  // [2][NCHAIN][NFP]
   static constexpr int W_B = X_B + (2 * NCHAIN * NFP * 4 + 15) / 16 * 16;  // [EPB][NPM1P][NW]
   static constexpr int GA_B = W_B + (NW * EPB * NPM1P * 4 + 15) / 16 * 16;  // [NP] uint4
@@ -109,7 +110,6 @@ struct FastLayout {
   // resident blocks per SM the register budget is sized for (2 when two tiles fit in the
   // shared memory of an SM, else 1)
   static constexpr int MINB = 2 * BYTES <= 227 * 1024 ? 2 : 1;
-  static_assert((EPB * NP * 4) % 16 == 0, "tile segments must be multiples of 16 bytes");
   static_assert(NFP < 255, "face node indices are packed in bytes");
   static_assert(NPM1P <= 1024 && NPS <= 1024, "w indices and stack slots fit the packed table");
   static_assert(TPE % 32 == 0 && TPE >= 32, "element threads come in whole warps");
@@ -169,6 +169,26 @@ __device__ __forceinline__ void l2_prefetch(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
+// Copies of 16 bytes and more need the field rows of a tile on 16-byte boundaries, which an
+// odd Np or an element count that is no multiple of four does not give. Such tiles are copied by
+// the chain threads instead, 1 or 2 floats at a time (cp.async), each thread arriving on the
+// barrier when its own copies have landed.
+__device__ __forceinline__ void copy_async(float* dst, const float* src, int n, int vec, int c,
+                                           int nc) {
+#pragma unroll 1
+  for (int i = c * vec; i < n; i += nc * vec) {
+    if (vec == 2)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s_addr(dst + i)), "l"(src + i)
+                   : "memory");
+    else
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s_addr(dst + i)), "l"(src + i)
+                   : "memory");
+  }
+}
+__device__ __forceinline__ void mbar_arrive_async(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(s_addr(bar)) : "memory");
+}
+
 // One face lift chain for compile-time N: x = chain input (NFP values, smem); g = the face's
 // volume stack with entries NCH apart, g[stack_slot<N>(c_ijk(N,i,j,d)) * NCH] = F_d(i,j) =
 // l_d E_d(i,j) (slots fold to immediates: the loops are unrolled). The
@@ -219,7 +239,11 @@ __device__ __forceinline__ void lift_chain(const float* x, float* g) {
   }
 }
 
-template <int N, int PHYS, int EPB, int TPE>
+// ANY: the element count is no multiple of EPB (the last tile is partial) or the field rows are
+// not all on 16-byte boundaries. A kernel of its own, because the extra paths cost the others
+// 2 to 17 % (instruction cache and the issuer's lead time: Maxwell N = 10, K = 24,576, 426 against
+// 528 us per stage).
+template <int N, int PHYS, int EPB, int TPE, bool ANY>
 __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
                                   FastLayout<N, PHYS, EPB, TPE>::MINB)
     stage_fast_kernel(FastStageParams P) {
@@ -250,60 +274,95 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   __shared__ int s_fail;
   const int tid = threadIdx.x;
   const int64_t K = P.K;
-  // this launch's tiles end at ntiles (the host guarantees K % EPB == 0)
-  const int64_t ntiles = P.tile_end > 0 ? P.tile_end : K / EPB;
+  // this launch's tiles end at ntiles; the mesh's last tile holds what is left of K (K < 2^27)
+  const int ntiles = P.tile_end > 0 ? (int)P.tile_end : ((int)K + EPB - 1) / EPB;
+  auto tile_ne = [=](int t) { return ANY ? min(EPB, (int)K - t * EPB) : EPB; };
   const uint32_t wlim = P.wait_iters ? P.wait_iters : (1u << 24);
   const bool stage = P.mode != 0;
   // element threads: element le, lane u within the element
   const int le = tid / TPE, u = tid - (tid / TPE) * TPE;
   const bool is_elem = tid < NTE;
+  // tiles that hold element le: without the last one where that ends before le
+  const int mytiles = ANY ? ((int)K + EPB - 1 - le) / EPB : ntiles;
 
   auto slot_q = [](int s) { return reinterpret_cast<float*>(smem + s * L::SLOT); };
-  auto slot_geo = [](int s) { return reinterpret_cast<float*>(smem + s * L::SLOT + L::QBYTES); };
+  auto slot_geo = [](int s) { return reinterpret_cast<float*>(smem + s * L::SLOT + L::GEO_O); };
   auto slot_conn = [](int s) {
-    return reinterpret_cast<int32_t*>(smem + s * L::SLOT + L::QBYTES + L::GEOBYTES);
+    return reinterpret_cast<int32_t*>(smem + s * L::SLOT + L::GEO_O + L::GEOBYTES);
   };
   const float* gq = P.q;
   const float* gres = P.res;
   const float* ggeo = P.geo;
   const int32_t* gconn = P.conn;
-  // tile t's q, geometry and connectivity -> slot s (thread 0 only). With `leave_out` (the
-  // test-only fault mode) the slot's barrier is armed but the copies are not issued, so that
-  // phase never completes and the bounded waits on it run out.
-  auto issue_main = [=](int64_t t, int s, bool leave_out = false) {
-    const int64_t e0 = t * EPB;
-    mbar_expect_tx(&bar[s], L::QBYTES + L::GEOBYTES + L::CONNBYTES);
-    if (leave_out) return;
+  const bool bulk = !ANY || NP % 4 == 0 || P.vec == 4;  // every field row starts on a 16-byte boundary
+  const bool issuer = tid == NTE;                      // the first chain thread
+  // Field rows of tile t -> dst: bulk copies (the issuer) or, off the 16-byte boundaries, narrow
+  // ones (all chain threads).
+  auto copy_rows = [=](float* dst, const float* src, int t, uint64_t* b) {
+    const int64_t e0 = (int64_t)t * EPB;
+    const int ne = tile_ne(t);
+    if (bulk && ne == EPB) {
 #pragma unroll
-    for (int m = 0; m < NF; ++m)
-      tma_load(slot_q(s) + m * EPB * NP, gq + ((size_t)m * K + e0) * NP, EPB * NP * 4, &bar[s]);
-    tma_load(slot_geo(s), ggeo + e0 * BB_GEO_STRIDE, L::GEOBYTES, &bar[s]);
-    tma_load(slot_conn(s), gconn + e0 * 4, L::CONNBYTES, &bar[s]);
+      for (int m = 0; m < NF; ++m)
+        tma_load(dst + m * EPB * NP, src + ((size_t)m * K + e0) * NP, EPB * NP * 4, b);
+    } else {
+#pragma unroll 1
+      for (int m = 0; m < NF; ++m) {
+        const float* row = src + ((size_t)m * K + e0) * NP;
+        if (bulk) tma_load(dst + m * EPB * NP, row, ne * NP * 4, b);
+        else copy_async(dst + m * EPB * NP, row, ne * NP, P.vec, tid - NTE, L::CHT);
+      }
+      if (!bulk) mbar_arrive_async(b);
+    }
   };
-  // tile t's q, geometry, connectivity and res -> L2, two tiles before they are copied in
-  auto prefetch_tile = [=](int64_t t) {
-    const int64_t e0 = t * EPB;
+  // tile t's q, geometry and connectivity -> slot s (the copying threads). With `leave_out`
+  // (the test-only fault mode) the slot's barrier is armed but the copies are not issued, so
+  // that phase never completes and the bounded waits on it run out.
+  auto issue_main = [=](int t, int s, bool leave_out = false) {
+    const int64_t e0 = (int64_t)t * EPB;
+    const int ne = tile_ne(t);
+    if (issuer)
+      mbar_expect_tx(&bar[s], (bulk ? NF * ne * NP * 4 : 0) + ne * (BB_GEO_STRIDE * 4 + 16));
+    if (leave_out) return;
+    copy_rows(slot_q(s), gq, t, &bar[s]);
+    if (issuer) {
+      tma_load(slot_geo(s), ggeo + e0 * BB_GEO_STRIDE, ne * BB_GEO_STRIDE * 4, &bar[s]);
+      tma_load(slot_conn(s), gconn + e0 * 4, ne * 16, &bar[s]);
+    }
+  };
+  auto issue_res = [=](int t) {
+    if (issuer) mbar_expect_tx(&bar[2], bulk ? NF * tile_ne(t) * NP * 4 : 0);
+    copy_rows(sRes, gres, t, &bar[2]);
+  };
+  // tile t's q, geometry, connectivity and res -> L2, two tiles before they are copied in (the
+  // issuer); rows off the 16-byte boundaries are rounded down to them, inside the buffer
+  auto prefetch_row = [=](const float* p, int n) {
+    if (bulk) {
+      l2_prefetch(p, n * 4);
+    } else {
+      const uintptr_t lo = (uintptr_t)p & ~(uintptr_t)15;
+      const uintptr_t hi = (uintptr_t)(p + n) & ~(uintptr_t)15;
+      if (hi > lo) l2_prefetch(reinterpret_cast<const void*>(lo), (uint32_t)(hi - lo));
+    }
+  };
+  auto prefetch_tile = [=](int t) {
+    if (tile_ne(t) != EPB) return;  // the partial last tile goes without
+    const int64_t e0 = (int64_t)t * EPB;
 #pragma unroll
     for (int m = 0; m < NF; ++m) {
-      l2_prefetch(gq + ((size_t)m * K + e0) * NP, EPB * NP * 4);
-      if (stage) l2_prefetch(gres + ((size_t)m * K + e0) * NP, EPB * NP * 4);
+      prefetch_row(gq + ((size_t)m * K + e0) * NP, EPB * NP);
+      if (stage) prefetch_row(gres + ((size_t)m * K + e0) * NP, EPB * NP);
     }
     l2_prefetch(ggeo + e0 * BB_GEO_STRIDE, L::GEOBYTES);
     l2_prefetch(gconn + e0 * 4, L::CONNBYTES);
   };
-  auto issue_res = [=](int64_t t) {
-    const int64_t e0 = t * EPB;
-    mbar_expect_tx(&bar[2], L::QBYTES);
-#pragma unroll
-    for (int m = 0; m < NF; ++m)
-      tma_load(sRes + m * EPB * NP, gres + ((size_t)m * K + e0) * NP, EPB * NP * 4, &bar[2]);
-  };
 
   if (tid == 0) {
     s_fail = 0;
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    mbar_init(&bar[2], 1);
+    const uint32_t arrivals = bulk ? 1 : 1 + L::CHT;
+    mbar_init(&bar[0], arrivals);
+    mbar_init(&bar[1], arrivals);
+    mbar_init(&bar[2], arrivals);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
@@ -380,17 +439,16 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     }
   }
   __syncthreads();
-  // the first two tiles of this block go to the two slots; the first chain thread issues
-  // every bulk copy and counts them per barrier (for the drain at the end)
-  const int64_t t0 = P.tile_begin + blockIdx.x;
-  const bool issuer = tid == NTE;
+  // the first two tiles of this block go to the two slots; the copying threads count the
+  // copies per barrier (for the drain at the end)
+  const int t0 = (int)P.tile_begin + (int)blockIdx.x, step = (int)gridDim.x;
   uint32_t iss0 = 0u, iss1 = 0u, iss2 = 0u;
-  if (issuer && t0 < ntiles) {
+  if ((bulk ? issuer : !is_elem) && t0 < ntiles) {
     issue_main(t0, 0);
     ++iss0;
     if (stage) issue_res(t0), ++iss2;
-    if (t0 + gridDim.x < ntiles) issue_main(t0 + gridDim.x, 1), ++iss1;
-    if (t0 + 2 * (int64_t)gridDim.x < ntiles) prefetch_tile(t0 + 2 * (int64_t)gridDim.x);
+    if (t0 + step < ntiles) issue_main(t0 + step, 1), ++iss1;
+    if (issuer && t0 + 2 * step < ntiles) prefetch_tile(t0 + 2 * step);
   }
   uint32_t ph = 0u;  // bit b: parity of the phase barrier b waits for next (element threads)
   const float rkA = P.rkA, rkB = P.rkB, dt = P.dt, tau = P.tau;
@@ -398,8 +456,8 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   const int ff = u / FT, fa0 = u - (u / FT) * FT;
 
   // interface flux of face ff of element le of tile t (q in slot s) -> chain inputs xbuf
-  auto flux_tile = [&](int64_t t, int s, float* xbuf) {
-    const int64_t e0 = t * EPB;
+  auto flux_tile = [&](int t, int s, float* xbuf) {
+    const int64_t e0 = (int64_t)t * EPB;
     const float* sQ = slot_q(s);
     const float* sGeo = slot_geo(s);
     const int32_t* sConn = slot_conn(s);
@@ -483,7 +541,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
       atomicOr(P.status, 2);
     }
     ph ^= 1u;
-    flux_tile(t0, 0, sX);
+    if (!ANY || t0 < mytiles) flux_tile(t0, 0, sX);
   }
   __syncthreads();
 
@@ -499,10 +557,10 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   const int grp = le / L::GS;
   volatile int* vfail = &s_fail;
   int it = 0;
-  for (int64_t tile = t0; tile < ntiles; tile += gridDim.x, ++it) {
+  for (int tile = t0; tile < ntiles; tile += step, ++it) {
     const int s = it & 1;
-    const int64_t e0 = tile * EPB;
-    const int64_t tnext = tile + gridDim.x;
+    const int64_t e0 = (int64_t)tile * EPB;
+    const int tnext = tile + step;
     float* sQ = slot_q(s);
     const float* sGeo = slot_geo(s);
     const int32_t* sConn = slot_conn(s);
@@ -512,7 +570,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     if (!is_elem) {
       if (it > 0) {
         for (int g = 0; g < NG; ++g) nbar_sync(1 + NG + g, GCOUNT);
-        if (issuer && !*vfail && (tnext < ntiles || stage)) {
+        if ((bulk ? issuer : true) && !*vfail && (tnext < ntiles || stage)) {
           fence_async_smem();  // order the generic-proxy reads before the copies
           if (tnext < ntiles) {
             issue_main(tnext, s ^ 1, P.fault == 1 && it == 1);
@@ -520,11 +578,11 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
             else ++iss1;
           }
           if (stage) issue_res(tile), ++iss2;
-          if (tnext + gridDim.x < ntiles) prefetch_tile(tnext + gridDim.x);
+          if (issuer && tnext + step < ntiles) prefetch_tile(tnext + step);
         }
       }
       const int c = tid - NTE;
-      if (!*vfail && c < NCHAIN)
+      if (!*vfail && c < NCHAIN)  // a partial tile's spare chains lift stale inputs, unused
         lift_chain<N, NCH>(sX + (s * NCHAIN + c) * NFP, sG + (c / NCH) * NPS * NCH + c % NCH);
       for (int g = 0; g < NG; ++g) nbar_arrive(1 + g, GCOUNT);
     } else if (it > 0 && (nbar_sync(1 + NG + grp, GCOUNT), *vfail)) {
@@ -532,10 +590,10 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     } else {
       // the tile after next: its outside-tile neighbour traces (one contiguous NF x Nfp block
       // per face) are pulled into L2 now, a whole tile ahead of its flux phase
-      const int64_t tpre = tnext + gridDim.x;
+      const int tpre = tnext + step;
       int32_t cpre = 0;
-      const bool pre = fa0 == 0 && tpre < ntiles && P.trace_in != nullptr;
-      if (pre) cpre = __ldg(gconn + (tpre * EPB + le) * 4 + ff);
+      const bool pre = fa0 == 0 && tpre < (ANY ? min(ntiles, mytiles) : ntiles) && P.trace_in != nullptr;
+      if (pre) cpre = __ldg(gconn + ((int64_t)tpre * EPB + le) * 4 + ff);
       const float* g = sGeo + le * BB_GEO_STRIDE;
       // barycentric weights of J d/dx, J d/dy, J d/dz: g_a = (rxJ, sxJ, txJ, -sum)/2; the
       // sum over a is formed as sum_{a<3} g_a (x_a - x_3), which cancels smooth data
@@ -597,7 +655,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
       if (pre) {
         const int64_t nb = (int64_t)((uint32_t)cpre >> 5);
         const int nfc = (cpre >> 3) & 3;
-        if (nb < K && (nb < tpre * EPB || nb >= (tpre + 1) * EPB)) {
+        if (nb < K && (nb < (int64_t)tpre * EPB || nb >= (int64_t)(tpre + 1) * EPB)) {
           // the bulk prefetch wants a 16-byte aligned start and size; a face block
           // (NF * NFP floats) need not be, so widen it to 16-byte boundaries. The trace
           // buffer starts on such a boundary and its length (16 K NF NFP bytes) is a
@@ -614,7 +672,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
           atomicOr(P.status, 2);
         }
         ph ^= 1u << (s ^ 1);
-        if (!*vfail) flux_tile(tnext, s ^ 1, sX + (s ^ 1) * NCHAIN * NFP);
+        if (!*vfail && (!ANY || tnext < mytiles)) flux_tile(tnext, s ^ 1, sX + (s ^ 1) * NCHAIN * NFP);
       }
       if (stage && !*vfail) {
         if (!mbar_wait(&bar[2], (ph >> 2) & 1u, wlim)) {
@@ -627,7 +685,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     if (is_elem) nbar_sync(1 + grp, GCOUNT);
 
     // ---- B. sum lift stacks + volume term, divide by J, LSRK update ------------------
-    if (is_elem && !*vfail) {
+    if (is_elem && (!ANY || tile < mytiles) && !*vfail) {
       const float* g = sGeo + le * BB_GEO_STRIDE;
       const float invJ = g[9];
       float nxf[4], nyf[4], nzf[4];
@@ -773,6 +831,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
       }
     }
   }
+  if (ANY && !is_elem && !bulk) asm volatile("cp.async.wait_all;" ::: "memory");
   if (issuer) {
     // let the copies this thread issued land before the block exits: immediate when the
     // element threads consumed them, bounded otherwise
@@ -862,10 +921,10 @@ VolGroups volume_groups() {
   return v;
 }
 
-template <int N, int PHYS, int EPB, int TPE>
-int launch_fast_t(const FastLaunch& fl, const FastStageParams& P0, cudaStream_t st) {
+template <int N, int PHYS, int EPB, int TPE, bool ANY>
+int launch_fast_any(const FastLaunch& fl, const FastStageParams& P0, cudaStream_t st) {
   using L = FastLayout<N, PHYS, EPB, TPE>;
-  auto kern = stage_fast_kernel<N, PHYS, EPB, TPE>;
+  auto kern = stage_fast_kernel<N, PHYS, EPB, TPE, ANY>;
   static const VolGroups vg = volume_groups<N, PHYS, TPE>();
   FastStageParams P = P0;
   for (int g = 0; g < 16; ++g) P.vstart[g] = vg.start[g], P.vlen[g] = vg.len[g];
@@ -885,14 +944,31 @@ int launch_fast_t(const FastLaunch& fl, const FastStageParams& P0, cudaStream_t 
       return BB_ERR_CUDA;
     if (fl.device >= 0 && fl.device < 64) per_sm_of[fl.device].store(per_sm);
   }
-  if (P.K % EPB != 0) return BB_ERR_ARG;
-  const int64_t tend = P.tile_end > 0 ? P.tile_end : P.K / EPB;
-  if (P.tile_begin < 0 || P.tile_begin >= tend || tend > P.K / EPB) return BB_ERR_ARG;
+  const int64_t tall = (P.K + EPB - 1) / EPB, tend = P.tile_end > 0 ? P.tile_end : tall;
+  if (P.tile_begin < 0 || P.tile_begin >= tend || tend > tall) return BB_ERR_ARG;
   const int64_t ntiles = tend - P.tile_begin;
   int64_t grid = (int64_t)per_sm * fl.num_sms;
   if (grid > ntiles) grid = ntiles;
   kern<<<(int)grid, L::NT, L::BYTES, st>>>(P);
   return cudaGetLastError() == cudaSuccess ? BB_OK : BB_ERR_CUDA;
+}
+
+template <int N, int PHYS, int EPB, int TPE>
+int launch_fast_t(const FastLaunch& fl, const FastStageParams& P0, cudaStream_t st) {
+  constexpr int NP = FastLayout<N, PHYS, EPB, TPE>::NP;
+  FastStageParams P = P0;
+  // widest copy (floats) that every field row of every tile is aligned for: rows start at
+  // multiples of EPB NP and of K NP floats
+  const uintptr_t base = (uintptr_t)P.q | (uintptr_t)P.res;
+  auto fits = [&](int v) {
+    return base % (4 * v) == 0 && (EPB * NP) % v == 0 && (P.K * NP) % v == 0;
+  };
+  P.vec = fits(4) ? 4 : fits(2) ? 2 : 1;
+  if (NP % 4 == 0 && P.vec != 4) return BB_ERR_ARG;  // the callers pass 16-byte-aligned buffers
+  if constexpr ((EPB * NP) % 4 == 0)
+    if (P.vec == 4 && P.K % EPB == 0)
+      return launch_fast_any<N, PHYS, EPB, TPE, false>(fl, P, st);
+  return launch_fast_any<N, PHYS, EPB, TPE, true>(fl, P, st);
 }
 
 }  // namespace bbfast

@@ -1,9 +1,8 @@
 // Registry of the compiled degree-specialised stage-kernel variants:
 // X(N, physics, elements per block, threads per element). The first variant matching a query
-// (and dividing the element count) is the default for that (N, physics), so each degree
-// lists its fastest tile on a 16^3 x 6 mesh first; the 2-element tiles at the end serve
-// meshes whose element count is not a multiple of the larger tiles. Each is instantiated in
-// one bbdg_stage_fast_v*.cu.
+// is the default for that (N, physics), so each degree lists its fastest tile on a 16^3 x 6
+// mesh first; the others are candidates of the autotuner. A mesh's last tile may be partial.
+// Each variant is instantiated in one bbdg_stage_fast_v*.cu.
 #pragma once
 #define BB_FAST_VARIANTS(X) \
   X(9, BB_WAVE, 4, 64) \

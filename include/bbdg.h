@@ -116,7 +116,7 @@ int bb_solver_create(bb_ctx* ctx, int physics, int N, int64_t K, int dtype,
 int bb_solver_destroy(bb_solver* s);
 /* Elements per thread block and threads per block of the stage kernels (0 = default).
  * FP32 solvers of some degrees have degree-specialised kernels (whole lift chains in
- * registers, bulk-copy pipelined tiles); those need K to be a multiple of the tile. */
+ * registers, tiles copied ahead); their last tile may be partial, so any K will do. */
 int bb_solver_set_tile(bb_solver* s, int elems_per_block, int threads);
 int bb_solver_get_tile(const bb_solver* s, int* elems_per_block, int* threads);
 /* Shared memory of one generic-kernel tile of epb elements (and whether it runs the

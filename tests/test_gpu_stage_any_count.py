@@ -1,0 +1,57 @@
+"""Degree-specialised stage kernels on element counts that are no multiple of their tile.
+
+The last tile of a mesh is then partial, and where the field rows do not start on 16-byte
+boundaries (an odd number of coefficients) tiles are copied 8 or 4 bytes at a time. The meshes
+are a periodic cube plus 0 to 3 lone elements whose faces meet each other, so that every
+remainder of K modulo 4 occurs; the reference is the generic kernel in FP64.
+"""
+import dataclasses
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def mesh_with_lone_elements(bb, n, extra):
+    """uniform_tet_mesh(n) and `extra` copies of its first element, face 0 of each meeting its
+    face 1 and face 2 its face 3 (orientation (0, 1, 2), an involution)."""
+    m = bb.uniform_tet_mesh(n)
+    K = m.K
+    nbr = np.concatenate([m.nbr, np.repeat(np.arange(K, K + extra)[:, None], 4, axis=1)])
+    nbf = np.concatenate([m.nbr_face, np.tile([[1, 0, 3, 2]], (extra, 1))])
+    ori = np.concatenate([m.orient, np.zeros((extra, 4), m.orient.dtype)])
+    geo = np.concatenate([m.geo, np.repeat(m.geo[:1], extra, axis=0)])
+    return dataclasses.replace(m, K=K + extra, nbr=nbr, nbr_face=nbf, orient=ori, geo=geo,
+                               conn=bb.mesh.pack_connectivity(nbr, nbf, ori))
+
+
+def rel(a, b):
+    return [float((x.double() - y).norm() / y.norm()) for x, y in zip(a, b)]
+
+
+# degrees with Np a multiple of 4 (bulk copies always), Np = 2 mod 4 and Np odd
+@pytest.mark.parametrize("physics,N", [("wave", 4), ("maxwell", 4), ("wave", 5), ("maxwell", 6),
+                                       ("wave", 8), ("maxwell", 8), ("wave", 9), ("maxwell", 10),
+                                       ("wave", 11)])
+@pytest.mark.parametrize("n,extra", [(2, 0), (2, 1), (2, 2), (2, 3), (7, 1)])
+def test_any_element_count(cuda, bb, physics, N, n, extra):
+    """The right-hand side of a random state and two LSRK steps against FP64: 1e-5 per field,
+    the repository's FP32 tolerance. K = 48 .. 51 is one or a few tiles, K = 2,059 (7^3 x 6 + 1)
+    several per block with a partial last one."""
+    import torch
+    m = mesh_with_lone_elements(bb, n, extra)
+    s = bb.DGSolver(m, N, physics, dtype=torch.float32, tau=1.0)
+    assert s.kernel == "specialised"
+    d = bb.DGSolver(m, N, physics, dtype=torch.float64, tau=1.0)
+    gen = torch.Generator(device=cuda).manual_seed(10 * N + extra)
+    q = torch.rand((s.nf, m.K, s.Np), generator=gen, device=cuda) * 2 - 1
+    q64 = q.double()
+    err = rel(s.rhs(q), d.rhs(q64))
+    assert max(err) < 1e-5, err
+    dt = s.dt_cfl()
+    s.run(q, torch.zeros_like(q), dt, 2)
+    s.check()
+    d.run(q64, torch.zeros_like(q64), dt, 2)
+    err = rel(q, q64)
+    assert max(err) < 1e-5, err
