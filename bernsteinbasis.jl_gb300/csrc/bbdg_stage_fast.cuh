@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+constexpr int BB_VOL_GROUPS = 32;  // warp-rounds of the volume phase
+
 struct FastStageParams {
   const uint32_t* gtab;  // degree tables (DegTables::d_words) and their word offsets
   int o_node3, o_node3m1, o_fvol, o_fperm, o_sslot;
@@ -23,8 +25,8 @@ struct FastStageParams {
   int vec;               // floats per copy the field rows are aligned for: 4 = bulk copies, 2, 1
   // volume phase: warp-round g = r * (TPE / 32) + warp forms w(beta) for beta = vstart[g] +
   // lane, lane < vlen[g] (filled by the launcher)
-  uint16_t vstart[16];
-  uint8_t vlen[16];
+  uint16_t vstart[BB_VOL_GROUPS];
+  uint8_t vlen[BB_VOL_GROUPS];
 };
 
 struct FastLaunch {

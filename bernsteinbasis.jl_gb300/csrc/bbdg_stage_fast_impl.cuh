@@ -60,6 +60,18 @@ struct FPhys<BB_MAXWELL> {
   static constexpr int NF = 6, NCH = 6, NW = 6;
 };
 
+// From degree 12 on the arithmetic is the generic kernel's, operation by operation, so that a
+// state does not depend on which kernel advanced it: there one step amplifies a difference in
+// the last bit to 1e-5 of the state (degree 15), where it stays below 1e-7 up to degree 11. The
+// extra product per stack entry costs 3 % (wave N = 15).
+__host__ __device__ constexpr bool generic_order(int N) { return N >= 12; }
+// a * b; in generic order a rounded product: where a following weight is the constant 1 the
+// compiler would otherwise turn fma(1, x, a * b) into fma(a, b, x).
+template <int N>
+__device__ __forceinline__ float prod(float a, float b) {
+  return generic_order(N) ? __fmul_rn(a, b) : a * b;
+}
+
 template <int N, int PHYS, int EPB, int TPE>
 struct FastLayout {
   static constexpr int NP = (N + 1) * (N + 2) * (N + 3) / 6;
@@ -107,9 +119,13 @@ struct FastLayout {
   static constexpr int NG = EPB / GS;
   static constexpr int GCOUNT = GS * TPE + CHT;  // threads at each hand-off
   static_assert(EPB % GS == 0 && 2 * NG <= 15, "named barriers 1..15 cover the groups");
-  // resident blocks per SM the register budget is sized for (2 when two tiles fit in the
-  // shared memory of an SM, else 1)
-  static constexpr int MINB = 2 * BYTES <= 227 * 1024 ? 2 : 1;
+  // resident blocks per SM the register budget is sized for: as many as fit in the SM's shared
+  // memory (each block takes 1 KB more than it asks for), up to the four that its 64 named
+  // barriers allow. A budget for two blocks left half the SM empty at the low degrees: Maxwell
+  // N = 4, K = 82,944, 238 -> 172 us per stage, N = 5 217 -> 182, N = 6 269 -> 206, wave N = 10
+  // 168 -> 135.
+  static constexpr int FITB = 228 * 1024 / (BYTES + 1024);
+  static constexpr int MINB = FITB < 1 ? 1 : FITB < 4 ? FITB : 4;
   static_assert(NFP < 255, "face node indices are packed in bytes");
   static_assert(NPM1P <= 1024 && NPS <= 1024, "w indices and stack slots fit the packed table");
   static_assert(TPE % 32 == 0 && TPE >= 32, "element threads come in whole warps");
@@ -198,16 +214,25 @@ __device__ __forceinline__ void mbar_arrive_async(uint64_t* bar) {
 template <int N, int NCH>
 __device__ __forceinline__ void lift_chain(const float* x, float* g) {
   constexpr int NFP = (N + 1) * (N + 2) / 2;
+  // The inputs enter row by row: the stencil of row j reads rows j - 1, j and j + 1, so from
+  // N = 12 on, where two full triangles would not fit in the registers, only three rows of X are
+  // live beside E (N = 15: 136 + 45 values).
   float X[NFP];
+  constexpr int AHEAD = N >= 12 ? 1 : N;  // rows of X loaded ahead of the stencil
 #pragma unroll
-  for (int m = 0; m < NFP; ++m) X[m] = x[m];
+  for (int m = 0; m < c_tri(N, AHEAD < N ? AHEAD : N + 1); ++m) X[m] = x[m];
   float E[NFP];
 #pragma unroll
   for (int j = 0; j <= N; ++j) {
+    if (AHEAD < N && j + 1 <= N) {
+#pragma unroll
+      for (int i = 0; i + j + 1 <= N; ++i) X[c_ij(N, i, j + 1)] = x[c_ij(N, i, j + 1)];
+    }
 #pragma unroll
     for (int i = 0; i + j <= N; ++i) {
       const int k = N - i - j;
-      float v = float((i + 1) * (i + 1) + (j + 1) * (j + 1) + (k + 1) * (k + 1)) * X[c_ij(N, i, j)];
+      float v = prod<N>(float((i + 1) * (i + 1) + (j + 1) * (j + 1) + (k + 1) * (k + 1)),
+                        X[c_ij(N, i, j)]);
       if (j > 0) v = fmaf(float((i + 1) * j), X[c_ij(N, i + 1, j - 1)], v);
       if (k > 0) v = fmaf(float((i + 1) * k), X[c_ij(N, i + 1, j)], v);
       if (i > 0) v = fmaf(float((j + 1) * i), X[c_ij(N, i - 1, j + 1)], v);
@@ -229,9 +254,14 @@ __device__ __forceinline__ void lift_chain(const float* x, float* g) {
       for (int i = 0; i + j < n; ++i) {
         // reduction_multiply! (src/BernsteinLift.jl:81-85) times l_d / l_{d-1}, in place in
         // ascending order
-        const float v = float(i + 1) * inv * E[c_ij(N, i + 1, j)] +
-                        (float(j + 1) * inv * E[c_ij(N, i, j + 1)] +
-                         float(n - i - j) * inv * E[c_ij(N, i, j)]);
+        const float v =
+            generic_order(N)
+                ? fmaf(float(i + 1), E[c_ij(N, i + 1, j)],
+                       fmaf(float(j + 1), E[c_ij(N, i, j + 1)],
+                            prod<N>(float(n - i - j), E[c_ij(N, i, j)]))) * inv
+                : float(i + 1) * inv * E[c_ij(N, i + 1, j)] +
+                      (float(j + 1) * inv * E[c_ij(N, i, j + 1)] +
+                       float(n - i - j) * inv * E[c_ij(N, i, j)]);
         E[c_ij(N, i, j)] = v;
         g[stack_slot<N>(c_ijk(N, i, j, d)) * NCH] = v;
       }
@@ -472,9 +502,15 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     float cp = 1.f, cu = 1.f;
     if (tau > 0.f) {
       const float n2 = nx * nx + ny * ny + nz * nz;
-      const float rJf = rsqrtf(n2);
-      cp = tau * n2 * rJf;  // tau |n|
-      cu = tau * rJf;       // tau / |n|
+      if constexpr (generic_order(N)) {
+        const float Jf = sqrtf(n2);
+        cp = tau * Jf;
+        cu = tau / Jf;
+      } else {
+        const float rJf = rsqrtf(n2);
+        cp = tau * n2 * rJf;  // tau |n|
+        cu = tau * rJf;       // tau / |n|
+      }
     }
     // outside-tile neighbour traces: issue every global load before using any
     float tr[FR][NF];
@@ -721,16 +757,17 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
 #pragma unroll
         for (int b = 0; b < 4; ++b)
           ab[b] = __uint_as_float(__byte_perm(ga.z, 0x4B000000u, 0x7540u + b)) - 8388608.0f;
-        // vol(alpha) = sum_b alpha_b w(alpha - e_b), b = 3 first (as the fma nesting before)
+        // vol(alpha) = sum_b alpha_b w(alpha - e_b), b = 3 first (b = 0 first in generic order)
+        constexpr int B0 = generic_order(N) ? 0 : 3, BS = generic_order(N) ? 1 : -1;
         float vol[NW];
         if constexpr (NW == 4) {
-          const float4 w3 = *reinterpret_cast<const float4*>(wb + xb[3] * 4);
-          vol[0] = ab[3] * w3.x;
-          vol[1] = ab[3] * w3.y;
-          vol[2] = ab[3] * w3.z;
-          vol[3] = ab[3] * w3.w;
+          const float4 w3 = *reinterpret_cast<const float4*>(wb + xb[B0] * 4);
+          vol[0] = ab[B0] * w3.x;
+          vol[1] = ab[B0] * w3.y;
+          vol[2] = ab[B0] * w3.z;
+          vol[3] = ab[B0] * w3.w;
 #pragma unroll
-          for (int b = 2; b >= 0; --b) {
+          for (int b = B0 + BS; b >= 0 && b <= 3; b += BS) {
             const float4 wv = *reinterpret_cast<const float4*>(wb + xb[b] * 4);
             vol[0] = fmaf(ab[b], wv.x, vol[0]);
             vol[1] = fmaf(ab[b], wv.y, vol[1]);
@@ -740,12 +777,12 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
         } else {
 #pragma unroll
           for (int m = 0; m < NW; m += 2) {
-            const float2 w3 = *reinterpret_cast<const float2*>(wb + xb[3] * NW + m);
-            vol[m] = ab[3] * w3.x;
-            vol[m + 1] = ab[3] * w3.y;
+            const float2 w3 = *reinterpret_cast<const float2*>(wb + xb[B0] * NW + m);
+            vol[m] = ab[B0] * w3.x;
+            vol[m + 1] = ab[B0] * w3.y;
           }
 #pragma unroll
-          for (int b = 2; b >= 0; --b) {
+          for (int b = B0 + BS; b >= 0 && b <= 3; b += BS) {
 #pragma unroll
             for (int m = 0; m < NW; m += 2) {
               const float2 wv = *reinterpret_cast<const float2*>(wb + xb[b] * NW + m);
@@ -759,8 +796,11 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
           // face order of src/BernsteinLift.jl:202-214: t=-1 face first, then f1, f2, f3;
           // the stacks already carry the l_d weights
           const float2 g3 = *reinterpret_cast<const float2*>(G + (3 * NPS + p[3]) * 2);
-          float A = g3.x;
-          float Bx = nxf[3] * g3.y, By = nyf[3] * g3.y, Bz = nzf[3] * g3.y;
+          constexpr bool GO = generic_order(N);  // the volume term first, then the faces
+          float A = GO ? g3.x - vol[0] : g3.x;
+          float Bx = GO ? fmaf(nxf[3], g3.y, -vol[1]) : nxf[3] * g3.y;
+          float By = GO ? fmaf(nyf[3], g3.y, -vol[2]) : nyf[3] * g3.y;
+          float Bz = GO ? fmaf(nzf[3], g3.y, -vol[3]) : nzf[3] * g3.y;
 #pragma unroll
           for (int f = 0; f < 3; ++f) {
             const float2 gf = *reinterpret_cast<const float2*>(G + (f * NPS + p[f]) * 2);
@@ -769,17 +809,17 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
             By = fmaf(nyf[f], gf.y, By);
             Bz = fmaf(nzf[f], gf.y, Bz);
           }
-          rhs[0] = (A - vol[0]) * invJ;
-          rhs[1] = (Bx - vol[1]) * invJ;
-          rhs[2] = (By - vol[2]) * invJ;
-          rhs[3] = (Bz - vol[3]) * invJ;
+          rhs[0] = (GO ? A : A - vol[0]) * invJ;
+          rhs[1] = (GO ? Bx : Bx - vol[1]) * invJ;
+          rhs[2] = (GO ? By : By - vol[2]) * invJ;
+          rhs[3] = (GO ? Bz : Bz - vol[3]) * invJ;
         } else {
           float v[6];
 #pragma unroll
           for (int m = 0; m < 6; m += 2) {
             const float2 g3 = *reinterpret_cast<const float2*>(G + (3 * NPS + p[3]) * 6 + m);
-            v[m] = g3.x;
-            v[m + 1] = g3.y;
+            v[m] = generic_order(N) ? vol[m] + g3.x : g3.x;
+            v[m + 1] = generic_order(N) ? vol[m + 1] + g3.y : g3.y;
           }
 #pragma unroll
           for (int f = 0; f < 3; ++f) {
@@ -791,7 +831,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
             }
           }
 #pragma unroll
-          for (int m = 0; m < 6; ++m) rhs[m] = (v[m] + vol[m]) * invJ;
+          for (int m = 0; m < 6; ++m) rhs[m] = (generic_order(N) ? v[m] : v[m] + vol[m]) * invJ;
         }
       }
       float* __restrict__ gq_out = P.q;
@@ -847,39 +887,28 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
 // beta + e_a (a = 0..3, 32 lanes, one word each) and the w(beta) store (NW floats per point, in
 // 16-byte or 8-byte pieces). Exact dynamic programme over the cut positions.
 struct VolGroups {
-  uint16_t start[16];
-  uint8_t len[16];
+  uint16_t start[BB_VOL_GROUPS];
+  uint8_t len[BB_VOL_GROUPS];
 };
 template <int N, int PHYS, int TPE>
 VolGroups volume_groups() {
   constexpr int NPM1 = N * (N + 1) * (N + 2) / 6, NF = FPhys<PHYS>::NF, NW = FPhys<PHYS>::NW;
   constexpr int VR = (NPM1 + TPE - 1) / TPE, G = VR * (TPE / 32);
-  static_assert(G <= 16 && NPM1 < 65536, "volume groups fit the launch parameters");
+  static_assert(G <= BB_VOL_GROUPS && NPM1 < 65536, "volume groups fit the launch parameters");
   std::vector<std::array<int, 4>> qi(NPM1);
   for (int k = 0, b = 0; k < N; ++k)
     for (int j = 0; j < N - k; ++j)
       for (int i = 0; i < N - j - k; ++i, ++b)
         qi[b] = {ijk3(N, i + 1, j, k), ijk3(N, i, j + 1, k), ijk3(N, i, j, k + 1), ijk3(N, i, j, k)};
-  // wavefronts of one access: per phase of `lanes` lanes, the largest number of distinct
-  // addresses (in units of `unit` words) that share a bank group
+  // wavefronts of one access (all addresses different): per phase of `lanes` lanes, the largest
+  // number of addresses (in units of `unit` words) that share a bank group
   auto wavefronts = [](const std::vector<int>& words, int unit, int lanes) {
     int tot = 0;
     const int groups = 32 / unit;
     for (size_t p0 = 0; p0 < words.size(); p0 += lanes) {
-      int best = 0;
-      for (int g = 0; g < groups; ++g) {
-        int cnt = 0;
-        std::vector<int> seen;
-        for (size_t q = p0; q < words.size() && q < p0 + lanes; ++q) {
-          const int a = words[q] / unit;
-          if (a % groups != g) continue;
-          bool dup = false;
-          for (int x : seen) dup |= x == a;
-          if (!dup) seen.push_back(a), ++cnt;
-        }
-        best = std::max(best, cnt);
-      }
-      tot += best;
+      std::array<int, 32> cnt{};
+      for (size_t q = p0; q < words.size() && q < p0 + lanes; ++q) ++cnt[words[q] / unit % groups];
+      tot += *std::max_element(cnt.begin(), cnt.end());
     }
     return tot;
   };
@@ -927,7 +956,7 @@ int launch_fast_any(const FastLaunch& fl, const FastStageParams& P0, cudaStream_
   auto kern = stage_fast_kernel<N, PHYS, EPB, TPE, ANY>;
   static const VolGroups vg = volume_groups<N, PHYS, TPE>();
   FastStageParams P = P0;
-  for (int g = 0; g < 16; ++g) P.vstart[g] = vg.start[g], P.vlen[g] = vg.len[g];
+  for (int g = 0; g < BB_VOL_GROUPS; ++g) P.vstart[g] = vg.start[g], P.vlen[g] = vg.len[g];
   P.wait_iters = fl.wait_iters;
   P.fault = fl.fault;
   // shared-memory opt-in and resident blocks per SM, set up once per device (the host-buffer

@@ -2,6 +2,7 @@
 // degrees so that the variants compile in parallel).
 #include "bbdg_stage_fast_impl.cuh"
 
+template int bbfast::launch_fast_t<7, BB_WAVE, 4, 32>(const FastLaunch&, const FastStageParams&, cudaStream_t);
 template int bbfast::launch_fast_t<7, BB_WAVE, 4, 64>(const FastLaunch&, const FastStageParams&, cudaStream_t);
 template int bbfast::launch_fast_t<7, BB_MAXWELL, 2, 64>(const FastLaunch&, const FastStageParams&, cudaStream_t);
 template int bbfast::launch_fast_t<8, BB_WAVE, 4, 64>(const FastLaunch&, const FastStageParams&, cudaStream_t);

@@ -31,7 +31,9 @@ def rel(a, b):
 
 
 # degrees with Np a multiple of 4 (bulk copies always), Np = 2 mod 4 and Np odd
-@pytest.mark.parametrize("physics,N", [("wave", 4), ("maxwell", 4), ("wave", 5), ("maxwell", 6),
+@pytest.mark.parametrize("physics,N", [("wave", 3), ("maxwell", 3), ("wave", 12), ("maxwell", 12),
+                                       ("wave", 13), ("maxwell", 13), ("wave", 14),
+                                       ("maxwell", 14), ("wave", 15), ("maxwell", 15), ("wave", 4), ("maxwell", 4), ("wave", 5), ("maxwell", 6),
                                        ("wave", 8), ("maxwell", 8), ("wave", 9), ("maxwell", 10),
                                        ("wave", 11)])
 @pytest.mark.parametrize("n,extra", [(2, 0), (2, 1), (2, 2), (2, 3), (7, 1)])
@@ -55,3 +57,26 @@ def test_any_element_count(cuda, bb, physics, N, n, extra):
     d.run(q64, torch.zeros_like(q64), dt, 2)
     err = rel(q, q64)
     assert max(err) < 1e-5, err
+
+
+@pytest.mark.parametrize("physics", ["wave", "maxwell"])
+@pytest.mark.parametrize("N", [12, 13, 14, 15])
+def test_high_degrees_equal_the_generic_kernel(cuda, bb, physics, N):
+    """From degree 12 on the specialised kernel does the generic kernel's arithmetic: the same
+    bits, in both penalty modes and with a partial last tile."""
+    import torch
+    m = mesh_with_lone_elements(bb, 3, 1)
+    for tau in (1.0, 0.0):
+        s = bb.DGSolver(m, N, physics, dtype=torch.float32, tau=tau)
+        assert s.kernel == "specialised"
+        gen = torch.Generator(device=cuda).manual_seed(N)
+        q0 = torch.rand((s.nf, m.K, s.Np), generator=gen, device=cuda) * 2 - 1
+        out = []
+        for kind in ("specialised", "generic"):
+            s.set_kernel(kind)
+            q = q0.clone()
+            rhs = s.rhs(q)
+            s.run(q, torch.zeros_like(q), 1e-3 * s.dt_cfl(), 2)
+            s.check()
+            out.append((rhs, q))
+        assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
