@@ -504,13 +504,7 @@ extern "C" int bb_rhs(bb_solver* s, const void* q, void* rhs, void* stream) {
   int rc = bb_set_device(s->ctx);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  const void* tin = nullptr;
-  if (s->fast >= 0) {  // the specialised kernel reads outside-tile traces from the buffer
-    rc = launch_extract(s, q, s->trace[0], st);
-    if (rc) return rc;
-    tin = s->trace[0];
-  }
-  rc = launch_stage(s, 0, 0, 0.0, const_cast<void*>(q), nullptr, rhs, tin, nullptr, st);
+  rc = launch_stage(s, 0, 0, 0.0, const_cast<void*>(q), nullptr, rhs, nullptr, nullptr, st);
   if (rc) return rc;
   return check_status(s, st);
 }

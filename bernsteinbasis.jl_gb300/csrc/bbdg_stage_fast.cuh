@@ -15,7 +15,8 @@ struct FastStageParams {
   float* q;              // [NF][K][Np]
   float* res;            // [NF][K][Np]
   float* rhs;            // mode 0 output
-  const float* trace_in; // [K][4][NF][Nfp], all faces that cross a tile boundary
+  const float* trace_in; // [K][4][NF][Nfp], all faces that cross a tile boundary; nullptr
+                         // (mode 0 only): neighbour nodes are read from q
   float* trace_out;      // [K][4][NF][Nfp] or nullptr
   const float* geo;      // [K][BB_GEO_STRIDE]
   const int32_t* conn;   // [K][4]

@@ -514,14 +514,29 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     }
     // outside-tile neighbour traces: issue every global load before using any
     float tr[FR][NF];
-    const float* tbase = P.trace_in + ((size_t)(bad ? 0 : nbr) * 4 + nface) * NF * NFP;
+    if (P.trace_in != nullptr) {
+      const float* tbase = P.trace_in + ((size_t)(bad ? 0 : nbr) * 4 + nface) * NF * NFP;
 #pragma unroll
-    for (int r = 0; r < FR; ++r) {
-      const int a = fa0 + r * FT;
-      if (a < NFP && !inside && !bad && BB_DCHECK(sFperm[o * NFP + a] < NFP, P.status)) {
-        const float* tp = tbase + sFperm[o * NFP + a];
+      for (int r = 0; r < FR; ++r) {
+        const int a = fa0 + r * FT;
+        if (a < NFP && !inside && !bad && BB_DCHECK(sFperm[o * NFP + a] < NFP, P.status)) {
+          const float* tp = tbase + sFperm[o * NFP + a];
 #pragma unroll
-        for (int m = 0; m < NF; ++m) tr[r][m] = __ldg(tp + m * NFP);
+          for (int m = 0; m < NF; ++m) tr[r][m] = __ldg(tp + m * NFP);
+        }
+      }
+    } else if (!inside && !bad) {
+      // a right-hand side alone leaves q unchanged: the neighbour's nodes come from q itself,
+      // without a launch (and a pass over the traces) to extract them first
+      const float* qn = gq + (size_t)nbr * NP;
+#pragma unroll
+      for (int r = 0; r < FR; ++r) {
+        const int a = fa0 + r * FT;
+        if (a < NFP && BB_DCHECK(sFnb[(nface * 6 + o) * NFP + a] < NP, P.status)) {
+          const float* tp = qn + sFnb[(nface * 6 + o) * NFP + a];
+#pragma unroll
+          for (int m = 0; m < NF; ++m) tr[r][m] = __ldg(tp + (size_t)m * K * NP);
+        }
       }
     }
     const int pin = (int)(nbr - e0);
