@@ -116,6 +116,7 @@ struct bb_batch {
   std::vector<const DegTables*> tabs;
   std::vector<int> epb;          // per problem
   std::vector<int> fast;         // per problem: specialised variant, -1 = generic kernel
+  std::vector<const void*> fast_tables;  // its table image
   int nfast = 0, ngeneric = 0;
   std::vector<void*> trace;      // 2 per problem
   void* d_desc = nullptr;
@@ -159,6 +160,7 @@ int build_desc(bb_batch* b) {
   const int np = (int)b->probs.size();
   auto a16 = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
   b->fast.assign(np, -1);
+  b->fast_tables.assign(np, nullptr);
   b->nfast = b->ngeneric = 0;
   for (int p = 0; p < np; ++p) {
     const bb_batch_problem& pr = b->probs[p];
@@ -169,7 +171,11 @@ int build_desc(bb_batch* b) {
       if (idx >= 0 && bb_fast_variant_info(idx, &e, &th, &sm) == BB_OK && sm <= ctx->smem_optin)
         b->fast[p] = idx;
     }
-    if (b->fast[p] >= 0) ++b->nfast;
+    if (b->fast[p] >= 0) {
+      b->fast_tables[p] = bb_fast_tables(ctx, b->fast[p]);
+      if (!b->fast_tables[p]) return bb_fail(ctx, BB_ERR_NOMEM, "table allocation failed");
+      ++b->nfast;
+    }
   }
   std::vector<BatchDesc<T>> h;
   int64_t begin = 0;
@@ -228,14 +234,8 @@ int build_desc(bb_batch* b) {
 // Stage s of a fast-lane problem: its specialised kernel, traces in buffer (par + s) & 1.
 int launch_fast_lane(bb_batch* b, int p, int s, int par, cudaStream_t st) {
   const bb_batch_problem& pr = b->probs[p];
-  const DegTables& t = *b->tabs[p];
   FastStageParams P{};
-  P.gtab = t.d_words;
-  P.o_node3 = t.o_node3;
-  P.o_node3m1 = t.o_node3m1;
-  P.o_fvol = t.o_fvol;
-  P.o_fperm = t.o_fperm;
-  P.o_sslot = t.o_sslot;
+  P.tables = b->fast_tables[p];
   P.K = pr.K;
   P.mode = 1;
   P.rkA = float(kA[s]);

@@ -71,7 +71,6 @@ struct DegTables {
   int o_fvol = 0;    // 4*Nfp uint16: face node -> volume index
   int o_fperm = 0;   // 6*Nfp uint16: face node -> neighbour face node, per orientation
   int o_fstack = 0;  // 4*Np uint16: face f's lift stack entry (layer, node) -> volume index
-  int o_sslot = 0;   // Np uint16: stage-kernel stack slot of lift-stack entry q (stack_slot<N>)
   int nwords = 0;
   uint32_t* d_words = nullptr;
 };
@@ -79,7 +78,7 @@ struct DegTables {
 // (shared-memory sizes of a tile are computed from it before the tables exist).
 inline int deg_table_words(int N) {
   return np3(N) + np3(N - 1) + (np3(N + 1) + 1) / 2 + (4 * np2(N) + 1) / 2 +
-         (6 * np2(N) + 1) / 2 + (4 * np3(N) + 1) / 2 + (np3(N) + 1) / 2;
+         (6 * np2(N) + 1) / 2 + (4 * np3(N) + 1) / 2;
 }
 
 // Orientation codes: face vertex m of this side is face vertex PERMS[o][m] of the partner,
@@ -102,6 +101,7 @@ struct bb_ctx {
   int64_t launches = 0;
   std::mutex mu;
   DegTables* tabs[BB_MAX_DEGREE + 2] = {};
+  std::vector<void*> fast_tabs;  // table images of the specialised stage kernels, by variant
   double* d_red = nullptr;     // reduction scratch (FP64 partials)
   size_t red_cap = 0;          // entries
   double* h_red = nullptr;     // pinned host mirror

@@ -8,7 +8,6 @@
 #include <cstring>
 
 #include "bbdg_internal.cuh"
-#include "bbdg_stack_slots.cuh"
 
 // -------------------------------------------------------------------------------------
 // context
@@ -96,6 +95,7 @@ extern "C" int bb_ctx_destroy(bb_ctx* ctx) {
   if (!ctx) return BB_ERR_ARG;
   cudaSetDevice(ctx->device);
   for (auto& t : ctx->tabs) free_tables(t);
+  for (void* t : ctx->fast_tabs) cudaFree(t);
   cudaFree(ctx->d_red);
   cudaFreeHost(ctx->h_red);
   cudaFree(ctx->d_status);
@@ -110,15 +110,6 @@ extern "C" const char* bb_ctx_last_error(const bb_ctx* ctx) {
 extern "C" int64_t bb_ctx_launch_count(const bb_ctx* ctx) { return ctx ? ctx->launches : -1; }
 
 // l_j(N) = (-1)^j C(N, j) / (1 + j)  (src/constants.jl:10-12)
-// Stage-kernel lift-stack slot of entry q (the generated tables of bbdg_stack_slots.cuh).
-static int stack_slot_of(int N, int q) {
-  switch (N) {
-    case 9: return stack_slot<9>(q);
-    case 10: return stack_slot<10>(q);
-    default: return q;
-  }
-}
-
 const DegTables* bb_tables(bb_ctx* ctx, int N) {
   if (!valid_degree(N)) return nullptr;
   std::lock_guard<std::mutex> lock(ctx->mu);
@@ -136,7 +127,6 @@ const DegTables* bb_tables(bb_ctx* ctx, int N) {
   t->o_fvol = off; off += (4 * t->Nfp + 1) / 2;
   t->o_fperm = off; off += (6 * t->Nfp + 1) / 2;
   t->o_fstack = off; off += (4 * t->Np + 1) / 2;
-  t->o_sslot = off; off += (t->Np + 1) / 2;
   t->nwords = off;
   if (off != deg_table_words(N)) {  // the tile-size estimates rely on the same count
     delete t;
@@ -183,7 +173,6 @@ const DegTables* bb_tables(bb_ctx* ctx, int N) {
       for (int b = 0; b <= N - d; ++b)
         for (int a = 0; a <= N - d - b; ++a) put16(t->o_fstack, f * t->Np + q++, face_vol(N, f, a, b, d));
   }
-  for (int q = 0; q < t->Np; ++q) put16(t->o_sslot, q, stack_slot_of(N, q));
   // (the lift weights l_j(N), constants.jl:10-12, are carried by the chain recursion:
   // no table of them is needed)
   bool ok = cudaMalloc(&t->d_words, sizeof(uint32_t) * off) == cudaSuccess &&

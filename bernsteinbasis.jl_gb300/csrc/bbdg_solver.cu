@@ -97,6 +97,7 @@ struct bb_solver {
   const DegTables* tab = nullptr;
   int epb = 0, threads = kThreads;
   int fast = -1;  // index of the degree-specialised FP32 variant in use, -1 = generic kernel
+  const void* fast_tables = nullptr;  // its table image (owned by the context)
   int generic_only = 0;
   int grid = 0;
   size_t smem = 0;
@@ -193,13 +194,7 @@ int launch_stage_t(bb_solver* s, int mode, int stage, double dt, void* q, void* 
 int launch_fast(bb_solver* s, int mode, int stage, double dt, void* q, void* res, void* rhs,
                 const void* tin, void* tout, cudaStream_t st, int64_t tb = 0, int64_t te = 0) {
   FastStageParams P;
-  const DegTables& t = *s->tab;
-  P.gtab = t.d_words;
-  P.o_node3 = t.o_node3;
-  P.o_node3m1 = t.o_node3m1;
-  P.o_fvol = t.o_fvol;
-  P.o_fperm = t.o_fperm;
-  P.o_sslot = t.o_sslot;
+  P.tables = s->fast_tables;
   P.K = s->K;
   P.tile_begin = tb;
   P.tile_end = te;
@@ -390,6 +385,11 @@ extern "C" int bb_solver_create(bb_ctx* ctx, int physics, int N, int64_t K, int 
     int e = 0, th = 0;
     size_t sm = 0;
     if (idx >= 0 && bb_fast_variant_info(idx, &e, &th, &sm) == BB_OK && sm <= ctx->smem_optin) {
+      s->fast_tables = bb_fast_tables(ctx, idx);
+      if (!s->fast_tables) {
+        delete s;
+        return bb_fail(ctx, BB_ERR_NOMEM, "table allocation failed");
+      }
       s->fast = idx;
       s->epb = e;
       s->threads = th;
@@ -441,8 +441,11 @@ extern "C" int bb_solver_set_tile(bb_solver* s, int epb, int threads) {
     int e = 0, th = 0;
     size_t sm = 0;
     if (idx >= 0 && bb_fast_variant_info(idx, &e, &th, &sm) == BB_OK && sm <= s->ctx->smem_optin) {
+      const void* tables = bb_fast_tables(s->ctx, idx);
+      if (!tables) return bb_fail(s->ctx, BB_ERR_NOMEM, "table allocation failed");
       if (idx != s->fast || e != s->epb) drop_graphs(s);
       s->fast = idx;
+      s->fast_tables = tables;
       s->epb = e;
       s->threads = th;
       s->smem = sm;

@@ -5,7 +5,7 @@
 
 using bbfast::FastLayout;
 #define BB_EXTERN(n_, p_, e_, t_) \
-  extern template int bbfast::launch_fast_t<n_, p_, e_, t_>(const FastLaunch&, const FastStageParams&, cudaStream_t);
+  extern template struct bbfast::FastKernel<n_, p_, e_, t_>;
 BB_FAST_VARIANTS(BB_EXTERN)
 #undef BB_EXTERN
 
@@ -55,10 +55,31 @@ extern "C" int bb_fast_variant(int idx, int* N, int* physics, int* epb, int* thr
   return BB_ERR_ARG;
 }
 
+const void* bb_fast_tables(bb_ctx* ctx, int idx) {
+  std::lock_guard<std::mutex> lock(ctx->mu);
+  if (idx < 0) return nullptr;
+  if ((size_t)idx >= ctx->fast_tabs.size()) ctx->fast_tabs.resize(idx + 1, nullptr);
+  void*& d = ctx->fast_tabs[idx];
+  if (d) return d;
+  std::vector<uint8_t> img;
+  int i = 0;
+#define BB_IMAGE(n_, p_, e_, t_)                                     \
+  if (idx == i) img = bbfast::FastKernel<n_, p_, e_, t_>::image();   \
+  ++i;
+  BB_FAST_VARIANTS(BB_IMAGE)
+#undef BB_IMAGE
+  if (img.empty() || cudaMalloc(&d, img.size()) != cudaSuccess) return d = nullptr;
+  if (cudaMemcpy(d, img.data(), img.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaFree(d);
+    d = nullptr;
+  }
+  return d;
+}
+
 int bb_fast_launch(int idx, const FastLaunch& fl, const FastStageParams& P, cudaStream_t st) {
   int i = 0;
 #define BB_LAUNCH(n_, p_, e_, t_)                                 \
-  if (idx == i) return bbfast::launch_fast_t<n_, p_, e_, t_>(fl, P, st);  \
+  if (idx == i) return bbfast::FastKernel<n_, p_, e_, t_>::launch(fl, P, st);  \
   ++i;
   BB_FAST_VARIANTS(BB_LAUNCH)
 #undef BB_LAUNCH

@@ -6,8 +6,7 @@
 constexpr int BB_VOL_GROUPS = 32;  // warp-rounds of the volume phase
 
 struct FastStageParams {
-  const uint32_t* gtab;  // degree tables (DegTables::d_words) and their word offsets
-  int o_node3, o_node3m1, o_fvol, o_fperm, o_sslot;
+  const void* tables;    // the variant's table image on the device (bb_fast_tables)
   int64_t K;
   int64_t tile_begin, tile_end;  // tiles [tile_begin, tile_end) of EPB elements (end 0 = all)
   int mode;              // 0: rhs only, 1: LSRK stage update
@@ -40,5 +39,9 @@ struct FastLaunch {
 // Index of the compiled variant for (N, physics, elements per block, threads), 0 = any; -1 if
 // none. Any element count will do: the last tile may be partial.
 int bb_fast_find(int N, int physics, int epb, int threads);
+// The variant's constant tables on the context's device, made on first use and freed with the
+// context; nullptr when out of memory. Not to be called while a stream is being captured.
+struct bb_ctx;
+const void* bb_fast_tables(bb_ctx* ctx, int idx);
 int bb_fast_variant_info(int idx, int* epb, int* threads, size_t* smem);
 int bb_fast_launch(int idx, const FastLaunch& fl, const FastStageParams& P, cudaStream_t st);

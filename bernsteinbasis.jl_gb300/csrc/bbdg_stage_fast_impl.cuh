@@ -111,7 +111,8 @@ struct FastLayout {
   static constexpr int FPERM_B = FVOL_B + ((4 * NFP * 2 + 3) / 4 * 4);  // [6][NFP] u16
   static constexpr int FNB_B = FPERM_B + ((6 * NFP * 2 + 3) / 4 * 4);  // [4][6][NFP] u16
   static constexpr int TF_B = (FNB_B + 24 * NFP * 2 + 15) / 16 * 16;   // [NP] u32 face nodes
-  static constexpr int BAR_B = (TF_B + NP * 4 + 15) / 16 * 16;         // 3 mbarriers
+  static constexpr int BAR_B = (TF_B + NP * 4 + 15) / 16 * 16;         // 4 mbarriers
+  static constexpr int TABLES = BAR_B - GA_B;  // the constant tables, one image (fast_image)
   static constexpr int BYTES = BAR_B + 32;
   // element groups for the named-barrier hand-offs between the chain warps and the element
   // threads: GS elements per group, NG groups, two barriers per group (ids 1..2 NG)
@@ -300,8 +301,10 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   uint16_t* sFnb = reinterpret_cast<uint16_t*>(smem + L::FNB_B);
   // per coefficient: its node index on faces f0..f3 (one byte each, 0xff = not on the face)
   uint32_t* sTF = reinterpret_cast<uint32_t*>(smem + L::TF_B);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_B);  // [0],[1] q slots, [2] res
+  uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_B);  // [0],[1] q slots, [2] res,
+                                                                 // [3] tables
   __shared__ int s_fail;
+  volatile int* vfail = &s_fail;
   const int tid = threadIdx.x;
   const int64_t K = P.K;
   // this launch's tiles end at ntiles; the mesh's last tile holds what is left of K (K < 2^27)
@@ -393,86 +396,21 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     mbar_init(&bar[0], arrivals);
     mbar_init(&bar[1], arrivals);
     mbar_init(&bar[2], arrivals);
+    mbar_init(&bar[3], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
-  // constant tables (built from the degree tables in global memory)
-  {
-    const uint32_t* gw = P.gtab;
-    // w index of alpha - e_b, or -1 when alpha_b = 0
-    auto wnb = [&](int n, int b) {
-      const uint32_t c = gw[P.o_node3 + n];
-      const int i = c & 0xff, j = (c >> 8) & 0xff, k = c >> 16, l = N - i - j - k;
-      const int ab = b == 0 ? i : b == 1 ? j : b == 2 ? k : l;
-      if (ab == 0) return -1;
-      return ijk3(N - 1, i - (b == 0), j - (b == 1), k - (b == 2));
-    };
-    auto group_of = [](int x) { return NW == 4 ? (x & 7) : ((3 * x) & 15); };
-    for (int t = tid; t < NP; t += NT) {
-      const uint32_t c = gw[P.o_node3 + t];
-      const int i = c & 0xff, j = (c >> 8) & 0xff, k = c >> 16, l = N - i - j - k;
-      uint32_t mb[4];
-      const int lane = (t % TPE) & 31, phase = L::NZ;  // lanes of one vector-load phase
-      const int n0 = t - (lane % phase);
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int x = wnb(t, b);
-        if (x >= 0) {
-          mb[b] = (uint32_t)x;
-          continue;
-        }
-        uint32_t used = 0;
-        for (int q = 0; q < phase; ++q) {
-          const int nq = n0 + q;
-          if (nq >= NP || (nq % TPE) / 32 != (t % TPE) / 32) continue;
-          const int xq = wnb(nq, b);
-          if (xq >= 0) used |= 1u << group_of(xq);
-        }
-        int zs = 0;
-        while (zs < L::NZ - 1 && ((used >> group_of(L::Z0 + zs)) & 1u)) ++zs;
-        mb[b] = (uint32_t)(L::Z0 + zs);
-      }
-      // stack slots of this coefficient on faces f0 (i,k,j), f1 (j,k,l), f2 (j,k,i), f3 (i,j,k)
-      // (the slot map is in the degree tables: no switch in the kernel's set-up code)
-      const uint16_t* gs = reinterpret_cast<const uint16_t*>(gw + P.o_sslot);
-      const uint32_t p0 = gs[ijk3(N, i, k, j)], p1 = gs[ijk3(N, j, k, l)];
-      const uint32_t p2 = gs[ijk3(N, j, k, i)], p3 = gs[t];
-      // 10-bit fields: .x w indices of alpha - e_b for b = 0..2, .y stack slots on f0..f2,
-      // .w stack slot on f3 and the w index for b = 3; .z alpha's barycentric indices
-      // (i, j, k, l), one byte each
-      sGA[t] = make_uint4(mb[0] | (mb[1] << 10) | (mb[2] << 20), p0 | (p1 << 10) | (p2 << 20),
-                          (uint32_t)i | ((uint32_t)j << 8) | ((uint32_t)k << 16) | ((uint32_t)l << 24),
-                          p3 | (mb[3] << 10));
-      // face nodes: f0 (j=0) at (i,k), f1 (l=0) at (j,k), f2 (i=0) at (j,k), f3 (k=0) at (i,j)
-      const uint32_t a0 = j == 0 ? (uint32_t)ij2(N, i, k) : 0xffu;
-      const uint32_t a1 = l == 0 ? (uint32_t)ij2(N, j, k) : 0xffu;
-      const uint32_t a2 = i == 0 ? (uint32_t)ij2(N, j, k) : 0xffu;
-      const uint32_t a3 = k == 0 ? (uint32_t)ij2(N, i, j) : 0xffu;
-      sTF[t] = a0 | (a1 << 8) | (a2 << 16) | (a3 << 24);
-    }
-    for (int t = tid; t < NPM1; t += NT) {
-      const uint32_t c = gw[P.o_node3m1 + t];
-      const int i = c & 0xff, j = (c >> 8) & 0xff, k = c >> 16;
-      sVN[t] = make_uint2(ijk3(N, i + 1, j, k) | (ijk3(N, i, j + 1, k) << 16),
-                          ijk3(N, i, j, k + 1) | (ijk3(N, i, j, k) << 16));
-    }
-    for (int t = tid; t < NZ_W; t += NT)
-      sW[((t / (L::NZ * NW)) * L::NPM1P + L::Z0 + (t / NW) % L::NZ) * NW + t % NW] = 0.f;
-    const uint16_t* gf = reinterpret_cast<const uint16_t*>(gw + P.o_fvol);
-    for (int t = tid; t < 4 * NFP; t += NT) sFvol[t] = gf[t];
-    const uint16_t* gp = reinterpret_cast<const uint16_t*>(gw + P.o_fperm);
-    for (int t = tid; t < 6 * NFP; t += NT) sFperm[t] = gp[t];
-    for (int t = tid; t < 24 * NFP; t += NT) {
-      const int fo = t / NFP, a = t - fo * NFP;
-      const uint16_t* gfv = reinterpret_cast<const uint16_t*>(gw + P.o_fvol);
-      sFnb[t] = gfv[(fo / 6) * NFP + gp[(fo % 6) * NFP + a]];
-    }
-  }
+  for (int t = tid; t < NZ_W; t += NT)
+    sW[((t / (L::NZ * NW)) * L::NPM1P + L::Z0 + (t / NW) % L::NZ) * NW + t % NW] = 0.f;
   __syncthreads();
   // the first two tiles of this block go to the two slots; the copying threads count the
   // copies per barrier (for the drain at the end)
   const int t0 = (int)P.tile_begin + (int)blockIdx.x, step = (int)gridDim.x;
   uint32_t iss0 = 0u, iss1 = 0u, iss2 = 0u;
+  if (issuer) {
+    mbar_expect_tx(&bar[3], L::TABLES);
+    tma_load(sGA, P.tables, L::TABLES, &bar[3]);
+  }
   if ((bulk ? issuer : !is_elem) && t0 < ntiles) {
     issue_main(t0, 0);
     ++iss0;
@@ -585,14 +523,14 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     }
   };
 
-  // prologue: flux of the first tile
+  // prologue: the tables (the chain warps read none of them), flux of the first tile
   if (is_elem && t0 < ntiles) {
-    if (!mbar_wait(&bar[0], 0u, wlim)) {
+    if (!mbar_wait(&bar[3], 0u, wlim) || !mbar_wait(&bar[0], 0u, wlim)) {
       s_fail = 1;
       atomicOr(P.status, 2);
     }
     ph ^= 1u;
-    if (!ANY || t0 < mytiles) flux_tile(t0, 0, sX);
+    if (!*vfail && (!ANY || t0 < mytiles)) flux_tile(t0, 0, sX);
   }
   __syncthreads();
 
@@ -606,7 +544,6 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   //     threads sync on it after forming w and the next tile's flux.
   constexpr int GCOUNT = L::GCOUNT, NG = L::NG;
   const int grp = le / L::GS;
-  volatile int* vfail = &s_fail;
   int it = 0;
   for (int tile = t0; tile < ntiles; tile += step, ++it) {
     const int s = it & 1;
@@ -890,6 +827,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   if (issuer) {
     // let the copies this thread issued land before the block exits: immediate when the
     // element threads consumed them, bounded otherwise
+    mbar_wait(&bar[3], 0u, wlim);
     if (iss0) mbar_wait(&bar[0], (iss0 - 1u) & 1u, wlim);
     if (iss1) mbar_wait(&bar[1], (iss1 - 1u) & 1u, wlim);
     if (iss2) mbar_wait(&bar[2], (iss2 - 1u) & 1u, wlim);
@@ -965,6 +903,90 @@ VolGroups volume_groups() {
   return v;
 }
 
+// The constant tables of a variant as they lie in shared memory from GA_B on, built once per
+// context on the host: every block of every launch copies them in one bulk copy (10 KB at wave
+// N = 9). Building them in each block took 4 us of the 10 us that a stage of a small mesh takes.
+template <int N, int PHYS, int EPB, int TPE>
+std::vector<uint8_t> fast_image() {
+  using L = FastLayout<N, PHYS, EPB, TPE>;
+  constexpr int NP = L::NP, NFP = L::NFP, NW = L::NW;
+  std::vector<uint8_t> img(L::TABLES, 0);
+  auto at = [&](int off) { return img.data() + (off - L::GA_B); };
+  uint32_t* ga = reinterpret_cast<uint32_t*>(at(L::GA_B));
+  uint32_t* vn = reinterpret_cast<uint32_t*>(at(L::VN_B));
+  uint16_t* fvol = reinterpret_cast<uint16_t*>(at(L::FVOL_B));
+  uint16_t* fperm = reinterpret_cast<uint16_t*>(at(L::FPERM_B));
+  uint16_t* fnb = reinterpret_cast<uint16_t*>(at(L::FNB_B));
+  uint32_t* tf = reinterpret_cast<uint32_t*>(at(L::TF_B));
+  std::vector<std::array<int, 4>> idx;
+  for (int k = 0; k <= N; ++k)
+    for (int j = 0; j <= N - k; ++j)
+      for (int i = 0; i <= N - j - k; ++i) idx.push_back({i, j, k, N - i - j - k});
+  // w index of alpha - e_b, or -1 when alpha_b = 0
+  auto wnb = [&](int n, int b) {
+    const std::array<int, 4>& a = idx[n];
+    return a[b] == 0 ? -1 : ijk3(N - 1, a[0] - (b == 0), a[1] - (b == 1), a[2] - (b == 2));
+  };
+  auto group_of = [](int x) { return NW == 4 ? (x & 7) : ((3 * x) & 15); };
+  for (int t = 0; t < NP; ++t) {
+    const int i = idx[t][0], j = idx[t][1], k = idx[t][2], l = idx[t][3];
+    uint32_t mb[4];
+    const int lane = (t % TPE) & 31, phase = L::NZ;  // lanes of one vector-load phase
+    const int n0 = t - (lane % phase);
+    for (int b = 0; b < 4; ++b) {
+      const int x = wnb(t, b);
+      if (x >= 0) {
+        mb[b] = (uint32_t)x;
+        continue;
+      }
+      uint32_t used = 0;
+      for (int nq = n0; nq < n0 + phase && nq < NP; ++nq) {
+        if ((nq % TPE) / 32 != (t % TPE) / 32) continue;
+        const int xq = wnb(nq, b);
+        if (xq >= 0) used |= 1u << group_of(xq);
+      }
+      int zs = 0;
+      while (zs < L::NZ - 1 && ((used >> group_of(L::Z0 + zs)) & 1u)) ++zs;
+      mb[b] = (uint32_t)(L::Z0 + zs);
+    }
+    // stack slots of this coefficient on faces f0 (i,k,j), f1 (j,k,l), f2 (j,k,i), f3 (i,j,k)
+    const uint32_t p0 = stack_slot<N>(ijk3(N, i, k, j)), p1 = stack_slot<N>(ijk3(N, j, k, l));
+    const uint32_t p2 = stack_slot<N>(ijk3(N, j, k, i)), p3 = stack_slot<N>(t);
+    // 10-bit fields: [0] w indices of alpha - e_b for b = 0..2, [1] stack slots on f0..f2, [3]
+    // stack slot on f3 and the w index for b = 3; [2] alpha's barycentric indices, one byte each
+    ga[4 * t] = mb[0] | (mb[1] << 10) | (mb[2] << 20);
+    ga[4 * t + 1] = p0 | (p1 << 10) | (p2 << 20);
+    ga[4 * t + 2] = (uint32_t)i | ((uint32_t)j << 8) | ((uint32_t)k << 16) | ((uint32_t)l << 24);
+    ga[4 * t + 3] = p3 | (mb[3] << 10);
+    // face nodes: f0 (j=0) at (i,k), f1 (l=0) at (j,k), f2 (i=0) at (j,k), f3 (k=0) at (i,j)
+    const uint32_t a0 = j == 0 ? (uint32_t)ij2(N, i, k) : 0xffu;
+    const uint32_t a1 = l == 0 ? (uint32_t)ij2(N, j, k) : 0xffu;
+    const uint32_t a2 = i == 0 ? (uint32_t)ij2(N, j, k) : 0xffu;
+    const uint32_t a3 = k == 0 ? (uint32_t)ij2(N, i, j) : 0xffu;
+    tf[t] = a0 | (a1 << 8) | (a2 << 16) | (a3 << 24);
+  }
+  for (int k = 0, t = 0; k < N; ++k)
+    for (int j = 0; j < N - k; ++j)
+      for (int i = 0; i < N - j - k; ++i, ++t) {
+        vn[2 * t] = ijk3(N, i + 1, j, k) | (ijk3(N, i, j + 1, k) << 16);
+        vn[2 * t + 1] = ijk3(N, i, j, k + 1) | (ijk3(N, i, j, k) << 16);
+      }
+  for (int b = 0, q = 0; b <= N; ++b)
+    for (int a = 0; a <= N - b; ++a, ++q) {
+      for (int f = 0; f < 4; ++f) fvol[f * NFP + q] = (uint16_t)face_vol(N, f, a, b, 0);
+      for (int o = 0; o < 6; ++o) {
+        const int wgt[3] = {a, b, N - a - b};
+        int wn[3];
+        for (int v = 0; v < 3; ++v) wn[perm_of(o, v)] = wgt[v];
+        fperm[o * NFP + q] = (uint16_t)ij2(N, wn[0], wn[1]);
+      }
+    }
+  for (int f = 0; f < 4; ++f)
+    for (int o = 0; o < 6; ++o)
+      for (int q = 0; q < NFP; ++q) fnb[(f * 6 + o) * NFP + q] = fvol[f * NFP + fperm[o * NFP + q]];
+  return img;
+}
+
 template <int N, int PHYS, int EPB, int TPE, bool ANY>
 int launch_fast_any(const FastLaunch& fl, const FastStageParams& P0, cudaStream_t st) {
   using L = FastLayout<N, PHYS, EPB, TPE>;
@@ -997,8 +1019,16 @@ int launch_fast_any(const FastLaunch& fl, const FastStageParams& P0, cudaStream_
   return cudaGetLastError() == cudaSuccess ? BB_OK : BB_ERR_CUDA;
 }
 
+// A compiled variant: its launch and its table image.
 template <int N, int PHYS, int EPB, int TPE>
-int launch_fast_t(const FastLaunch& fl, const FastStageParams& P0, cudaStream_t st) {
+struct FastKernel {
+  static int launch(const FastLaunch& fl, const FastStageParams& P, cudaStream_t st);
+  static std::vector<uint8_t> image() { return fast_image<N, PHYS, EPB, TPE>(); }
+};
+
+template <int N, int PHYS, int EPB, int TPE>
+int FastKernel<N, PHYS, EPB, TPE>::launch(const FastLaunch& fl, const FastStageParams& P0,
+                                          cudaStream_t st) {
   constexpr int NP = FastLayout<N, PHYS, EPB, TPE>::NP;
   FastStageParams P = P0;
   // widest copy (floats) that every field row of every tile is aligned for: rows start at
