@@ -72,6 +72,10 @@ struct DegTables {
   int o_fperm = 0;   // 6*Nfp uint16: face node -> neighbour face node, per orientation
   int o_fstack = 0;  // 4*Np uint16: face f's lift stack entry (layer, node) -> volume index
   int nwords = 0;
+  // past the nwords that blocks copy to shared memory:
+  int o_gather = 0;  // Np x 4: per coefficient the degree N-1 indices of alpha - e_b (b = 0..3)
+                     // and its positions in the lift stacks of faces 0..3, 16 bits each
+  int o_wred = 0;    // (N+1) x (N+2) doubles: -v / (d+1), the lift recursion's weights of layer d
   uint32_t* d_words = nullptr;
 };
 // 32-bit words of the degree-N tables, the sum of the DegTables sections above in order
@@ -305,6 +309,38 @@ __device__ __forceinline__ T finish_half(T v) {
   else return T(0.5) * v;
 }
 
+// The Maxwell interface flux of one face node (3d_maxwell.jl:52-63) from the jumps d, the scaled
+// normal n and the penalty weights: out = 0.5 (n x d terms) + 0.5 cp d - 0.5 cu n (n.d), four
+// operations per component with the halves folded into n and the weights (exact). Written out
+// with the zero entries of the example's coefficient arrays it was about 13 per component, which
+// no compiler may drop (0 x is not 0 for an infinite x).
+template <class T>
+__device__ __forceinline__ void maxwell_flux(const T (&d)[6], T nx, T ny, T nz, T cp, T cu,
+                                             T (&out)[6]) {
+  const T hx = T(0.5) * nx, hy = T(0.5) * ny, hz = T(0.5) * nz, hp = T(0.5) * cp;
+  const T tH = cu * fma(hz, d[2], fma(hy, d[1], hx * d[0]));
+  const T tE = cu * fma(hz, d[5], fma(hy, d[4], hx * d[3]));
+  out[0] = fma(hz, d[4], fma(-hy, d[5], fma(hp, d[0], -tH * nx)));
+  out[1] = fma(hx, d[5], fma(-hz, d[3], fma(hp, d[1], -tH * ny)));
+  out[2] = fma(hy, d[3], fma(-hx, d[4], fma(hp, d[2], -tH * nz)));
+  out[3] = fma(hy, d[2], fma(-hz, d[1], fma(hp, d[3], -tE * nx)));
+  out[4] = fma(hz, d[0], fma(-hx, d[2], fma(hp, d[4], -tE * ny)));
+  out[5] = fma(hx, d[1], fma(-hy, d[0], fma(hp, d[5], -tE * nz)));
+}
+
+// Adds the curl terms of one barycentric direction to the Maxwell w (J dH/dt = -curl E,
+// J dE/dt = curl H), two operations per component.
+template <class T>
+__device__ __forceinline__ void maxwell_curl(T (&w)[6], T gx, T gy, T gz, T Hx, T Hy, T Hz, T Ex,
+                                             T Ey, T Ez) {
+  w[0] = fma(gz, Ey, fma(-gy, Ez, w[0]));
+  w[1] = fma(gx, Ez, fma(-gz, Ex, w[1]));
+  w[2] = fma(gy, Ex, fma(-gx, Ey, w[2]));
+  w[3] = fma(gy, Hz, fma(-gz, Hy, w[3]));
+  w[4] = fma(gz, Hx, fma(-gx, Hz, w[4]));
+  w[5] = fma(gx, Hy, fma(-gy, Hx, w[5]));
+}
+
 // L0 x at face node (i, j) of degree N, k = N - i - j: the 7-point stencil of
 // (N+1)^2/2 R_{N+1} E_{N->N+1} (src/BernsteinLift.jl:100-125 then :66-90 with the L0
 // scaling), x in the 2D layout of degree N with row offsets rb (row j), rbn (row j+1) and
@@ -337,6 +373,50 @@ template <class T>
 __device__ __forceinline__ T reduce_point(int i, int j, int n, T x_ip, T x_jp, T x_0, T scale) {
   return fma(small_int<T>(i + 1), x_ip, fma(small_int<T>(j + 1), x_jp, small_int<T>(n - i - j) * x_0)) *
          scale;
+}
+
+// The face lifts of `nchain` chains at once, every layer kept: chain c's Nfp inputs at X + c xs,
+// its stack (layer d outer, then j, then i) at G + c gs. Level-parallel, one thread per entry and
+// a block barrier per layer; layer d is formed from layer d-1 where it lies in the stack, so all
+// faces of a tile take N+1 barriers together. The same recursion as lift_face_accumulate, in
+// double with the weights -v/(d+1) from a table (wred, row d of N+2) instead of integer weights
+// and a final product: three operations of the scarce FP64 pipe per entry instead of four.
+template <class T>
+__device__ void lift_stacks(int N, int nchain, const uint16_t* node2, const T* X, int xs, T* G,
+                            int gs, const T* wred) {
+  const int S = np2(N);
+  {
+    const uint16_t* dec = node2 + np3(N - 1);
+    const FastDiv by_s(S);
+    for (int it = threadIdx.x; it < nchain * S; it += blockDim.x) {
+      const int ch = by_s.div(it), m = it - ch * S;
+      const int a = dec[m] & 0xff, b = dec[m] >> 8, c = N - a - b;
+      const int rb = tri_off(N, b);
+      G[ch * gs + m] = l0_point<T>(a, b, c, X + ch * xs, rb, rb + (N + 1 - b), rb - (N + 2 - b));
+    }
+  }
+  __syncthreads();
+  int off = 0;  // layer d - 1 within a stack
+  for (int d = 1; d <= N; ++d) {
+    const int n = N + 1 - d;  // input degree
+    const int cnt = np2(n - 1), next = off + np2(n);
+    const uint16_t* dec = node2 + np3(n - 2);
+    const FastDiv by_cnt(cnt);
+    for (int it = threadIdx.x; it < nchain * cnt; it += blockDim.x) {
+      const int ch = by_cnt.div(it), m = it - ch * cnt;
+      const int a = dec[m] & 0xff, b = dec[m] >> 8;
+      T* g = G + ch * gs;
+      const T* x = g + off + ij2(n, a, b);  // (a, b); (a+1, b) and (a, b+1) at x[1], x[n+1-b]
+      if constexpr (sizeof(T) == 8) {
+        const T* w = wred + d * (N + 2);
+        g[next + m] = fma(w[a + 1], x[1], fma(w[b + 1], x[n + 1 - b], w[n - a - b] * x[0]));
+      } else {
+        g[next + m] = reduce_point<T>(a, b, n, x[1], x[n + 1 - b], x[0], -inv_int<T>(d + 1));
+      }
+    }
+    off = next;
+    __syncthreads();
+  }
 }
 
 // One face's recursive lift, accumulated into a shared-memory volume block, for `ne`

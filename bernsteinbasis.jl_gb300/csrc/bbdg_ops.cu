@@ -128,7 +128,10 @@ const DegTables* bb_tables(bb_ctx* ctx, int N) {
   t->o_fperm = off; off += (6 * t->Nfp + 1) / 2;
   t->o_fstack = off; off += (4 * t->Np + 1) / 2;
   t->nwords = off;
-  if (off != deg_table_words(N)) {  // the tile-size estimates rely on the same count
+  off = (off + 3) & ~3;
+  t->o_gather = off; off += 4 * t->Np;
+  t->o_wred = off; off += 2 * (N + 1) * (N + 2);
+  if (t->nwords != deg_table_words(N)) {  // the tile-size estimates rely on the same count
     delete t;
     return nullptr;
   }
@@ -173,6 +176,25 @@ const DegTables* bb_tables(bb_ctx* ctx, int N) {
       for (int b = 0; b <= N - d; ++b)
         for (int a = 0; a <= N - d - b; ++a) put16(t->o_fstack, f * t->Np + q++, face_vol(N, f, a, b, d));
   }
+  m = 0;
+  for (int k = 0; k <= N; ++k)
+    for (int j = 0; j <= N - k; ++j)
+      for (int i = 0; i <= N - j - k; ++i, ++m) {
+        const int l = N - i - j - k, at = 2 * t->o_gather + 8 * m;
+        put16(0, at, i > 0 ? ijk3(N - 1, i - 1, j, k) : 0);
+        put16(0, at + 1, j > 0 ? ijk3(N - 1, i, j - 1, k) : 0);
+        put16(0, at + 2, k > 0 ? ijk3(N - 1, i, j, k - 1) : 0);
+        put16(0, at + 3, l > 0 ? ijk3(N - 1, i, j, k) : 0);
+        put16(0, at + 4, ijk3(N, i, k, j));
+        put16(0, at + 5, ijk3(N, j, k, l));
+        put16(0, at + 6, ijk3(N, j, k, i));
+        put16(0, at + 7, m);
+      }
+  for (int d = 0; d <= N; ++d)
+    for (int v = 0; v <= N + 1; ++v) {
+      const double x = -(double)v / (double)(d + 1);
+      std::memcpy(w.data() + t->o_wred + 2 * (d * (N + 2) + v), &x, sizeof(x));
+    }
   // (the lift weights l_j(N), constants.jl:10-12, are carried by the chain recursion:
   // no table of them is needed)
   bool ok = cudaMalloc(&t->d_words, sizeof(uint32_t) * off) == cudaSuccess &&

@@ -18,7 +18,7 @@ namespace {
 constexpr int kThreads = 256;
 
 template <class T, int PHYS>
-__global__ void __launch_bounds__(kThreads) stage_kernel(StageParams<T> P, TileLayout L) {
+__global__ void __launch_bounds__(2 * kThreads, 2) stage_kernel(StageParams<T> P, TileLayout L) {
   extern __shared__ __align__(16) unsigned char smem[];
   const SmemTables st =
       load_tables(P.tab, P.gtab, reinterpret_cast<uint32_t*>(smem + L.tab_bytes));
@@ -149,6 +149,27 @@ int solver_layout(bb_solver* s, int epb, size_t* smem_out, int* chain_out = null
   return L.total <= s->ctx->smem_optin ? BB_OK : BB_ERR_ARG;
 }
 
+// Default tile of the FP64 kernel with whole stacks (0: none fits). Its time is what the busiest
+// SM takes, tiles per SM times the elements of a tile plus a set-up worth about 150 coefficients
+// per tile (measured: wave N = 7, K = 4,374, 151 / 136 / 131 us per stage at 1 / 2 / 3 elements,
+// N = 3, K = 10,368, 171 / 109 / 85 / 70 / 68 at 1 / 2 / 3 / 6 / 8); tiles of several elements
+// count only where three blocks fit on an SM (Maxwell N = 7, K = 4,374: 301 / 305 / 360 at 1 / 2 / 3
+// elements, 4 / 2 / 1 blocks) and every SM gets two tiles (wave N = 7, K = 384: 22 / 26 us).
+int stack_tile(bb_solver* s) {
+  int best = 0;
+  double cost = 0.0;
+  for (int e : {1, 2, 3, 4, 6, 8}) {
+    const TileLayout L = tile_layout_for(s->N, s->nf, physics_nw(s->physics), sizeof(double),
+                                         s->tab->nwords, e);
+    if (!L.stacks || L.total > s->ctx->smem_optin) continue;
+    const int64_t tiles = (s->K + e - 1) / e, sms = s->ctx->num_sms;
+    if (e > 1 && (3 * (L.total + 1024) > 228 * 1024 || tiles < 2 * sms)) continue;
+    const double c = (double)((tiles + sms - 1) / sms) * (e + 150.0 / (s->nf * s->tab->Np));
+    if (!best || c <= cost) best = e, cost = c;
+  }
+  return best;
+}
+
 // tb, te: the launch covers tiles [tb, te) of the solver's tile size (te = 0: all tiles).
 template <class T, int PHYS>
 int launch_stage_t(bb_solver* s, int mode, int stage, double dt, void* q, void* res, void* rhs,
@@ -187,7 +208,9 @@ int launch_stage_t(bb_solver* s, int mode, int stage, double dt, void* q, void* 
   if (ntiles < 1) return bb_fail(ctx, BB_ERR_ARG, "empty tile range");
   int64_t grid = (int64_t)per_sm * ctx->num_sms;
   if (grid > ntiles) grid = ntiles;
-  stage_kernel<T, PHYS><<<(int)grid, kThreads, L.total, st>>>(P, L);
+  // where the tile leaves room for one block per SM only, that block takes twice the threads
+  const int threads = per_sm == 1 ? 2 * kThreads : kThreads;
+  stage_kernel<T, PHYS><<<(int)grid, threads, L.total, st>>>(P, L);
   return bb_check_launch(ctx, "stage_kernel");
 }
 
@@ -358,8 +381,10 @@ extern "C" int bb_solver_create(bb_ctx* ctx, int physics, int N, int64_t K, int 
   s->tab = t;
   // default tile: the largest of 12, 6, 4, 2 elements whose tile runs the chain lift (FP32
   // tiles that fit its shared-memory budget); else, in this order, 4, 2, 6, 12 or 1 elements
-  // within 100 KB (FP64 always lifts level-parallel: wave N = 9 takes 2 elements)
+  // within 100 KB; FP64 with whole stacks has its own rule
   const int cands[2][5] = {{12, 6, 4, 2, 0}, {4, 2, 6, 12, 1}};
+  if (dtype == BB_F64) s->epb = stack_tile(s);
+  if (s->epb) solver_layout(s, s->epb, &s->smem);
   for (int pass = 0; pass < 2 && !s->epb; ++pass)
     for (int c : cands[pass]) {
       size_t sm = 0;

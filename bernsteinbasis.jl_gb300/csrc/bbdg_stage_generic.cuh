@@ -75,10 +75,12 @@ struct StageParams {
 // Shared-memory layout of a tile (in units of T unless noted). chain != 0: the lift runs one
 // thread per (element, face, chain) with the face stacks in shared memory (FP32 tiles that fit
 // in kChainLiftBytes); chain == 0: the level-parallel lift with two ping-pong rows.
+// stacks != 0: every chain of the tile keeps its whole stack (lift_stacks), and the gather, the
+// volume term and the update are one pass (`out` and the weights of lift_stacks share an offset).
 struct TileLayout {
-  size_t q, out, flux, work, geo, pen, gh, conn_bytes, tab_bytes, total;
+  size_t q, out, flux, work, stack, geo, pen, gh, conn_bytes, tab_bytes, total;
   int work_elems;
-  int chain;
+  int chain, stacks;
 };
 constexpr size_t kChainLiftBytes = 100 * 1024;
 // The batched kernel uses the same rule, so that a tile timed on a single problem (how its
@@ -114,16 +116,49 @@ __host__ __device__ inline TileLayout tile_layout_with(int N, int NF, int NW, si
   L.tab_bytes = bytes; bytes += (size_t)nwords * 4;
   L.total = align16(bytes);
   L.chain = chain;
+  L.stack = 0;
+  L.stacks = 0;
+  return L;
+}
+
+// The layout with whole stacks (row stride Np | 1, against bank conflicts).
+__host__ __device__ inline TileLayout tile_layout_stacks(int N, int NF, int NW, size_t tsize,
+                                                        int nwords, int epb) {
+  TileLayout L;
+  const size_t Np = np3(N), Nfp = np2(N), NpM1 = np3(N - 1);
+  const size_t nch = (size_t)lift_chains(NF);
+  size_t off = 0;
+  L.q = off; off += (size_t)NF * epb * Np;
+  L.flux = off; off += (size_t)epb * 4 * nch * Nfp;
+  L.work = off; off += (size_t)NW * epb * NpM1;
+  L.work_elems = (int)(NW * epb * NpM1);
+  L.stack = off; off += (size_t)epb * 4 * nch * (Np | 1);
+  L.geo = off; off += (size_t)epb * BB_GEO_STRIDE;
+  L.pen = off; off += (size_t)epb * 8;
+  L.gh = off; off += (size_t)epb * 9;
+  L.out = off; off += tsize == 8 ? (size_t)(N + 1) * (N + 2) : 0;  // wred
+  size_t bytes = align16(off * tsize);
+  L.conn_bytes = bytes; bytes += align16((size_t)epb * 4 * sizeof(int32_t));
+  L.tab_bytes = bytes; bytes += (size_t)nwords * 4;
+  L.total = align16(bytes);
+  L.chain = 0;
+  L.stacks = 1;
   return L;
 }
 
 // FP32: the chain lift when its tile fits in `budget` bytes, else the level-parallel one.
-// FP64 always takes the level-parallel lift: the chain phase keeps one thread per (element,
-// face, chain) busy, too few to feed the FP64 pipe (wave N = 9, 2-element tiles: the pipe is
-// 48 % busy with chains against 80 % level-parallel, 2.38 against 1.65 ms per stage).
+// FP64 always lifts level by level: the chain phase keeps one thread per (element, face, chain)
+// busy, too few to feed the FP64 pipe (wave N = 9, 2-element tiles: the pipe is 48 % busy with
+// chains against 80 % level-parallel, 2.38 against 1.65 ms per stage); with whole stacks
+// where they fit.
+constexpr size_t kStackBytes = 224 * 1024;
 __host__ __device__ inline TileLayout tile_layout_for(int N, int NF, int NW, size_t tsize,
                                                      int nwords, int epb,
                                                      size_t budget = kChainLiftBytes) {
+  if (tsize == 8) {
+    const TileLayout s = tile_layout_stacks(N, NF, NW, tsize, nwords, epb);
+    if (s.total <= kStackBytes) return s;
+  }
   const TileLayout c = tile_layout_with(N, NF, NW, tsize, nwords, epb, 1);
   return tsize == 4 && c.total <= budget ? c : tile_layout_with(N, NF, NW, tsize, nwords, epb, 0);
 }
@@ -174,6 +209,25 @@ TileLayout tile_layout(const DegTables& t, int epb) {
   return tile_layout_for(t.N, Phys<PHYS>::NF, Phys<PHYS>::NW, sizeof(T), t.nwords, epb);
 }
 
+// The traces of the tile's faces whose neighbour lies outside it, from the updated q in sQ.
+template <class T, int NF>
+__device__ void write_traces(const StageParams<T>& P, const SmemTables& st, const T* sQ,
+                             const int32_t* sConn, int64_t e0, int ne) {
+  const int Np = P.tab.Np, Nfp = P.tab.Nfp, epb = P.epb;
+  const FastDiv by_nfp(Nfp), by_nfnfp(NF * Nfp), by_4nfnfp(4 * NF * Nfp);
+  for (int it = threadIdx.x; it < ne * 4 * NF * Nfp; it += blockDim.x) {
+    const int le = by_4nfnfp.div(it);
+    int rem = it - le * 4 * NF * Nfp;
+    const int f = by_nfnfp.div(rem);
+    rem -= f * NF * Nfp;
+    const int fld = by_nfp.div(rem), a = rem - fld * Nfp;
+    const int64_t nbr = (int64_t)((uint32_t)sConn[le * 4 + f] >> 5);
+    if (nbr >= e0 && nbr < e0 + ne) continue;  // neighbour inside the tile
+    P.trace_out[((size_t)(e0 + le) * 4 + f) * NF * Nfp + (size_t)fld * Nfp + a] =
+        sQ[((size_t)fld * epb + le) * Np + st.fvol[f * Nfp + a]];
+  }
+}
+
 // One tile of the generic stage (all threads of the block call it). The degree tables are in
 // shared memory (st); the layout L matches P's degree, physics and tile.
 template <class T, int PHYS, bool CHAIN_LIFT = true>
@@ -193,8 +247,7 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
   const int N = P.tab.N, Np = P.tab.Np, NpM1 = P.tab.NpM1, Nfp = P.tab.Nfp;
   const int64_t K = P.K;
   const int epb = P.epb;
-  const FastDiv by_np(Np), by_npm1(NpM1), by_nfp(Nfp), by_4nfp(4 * Nfp), by_nfnp(NF * Np),
-      by_nfnfp(NF * Nfp), by_4nfnfp(4 * NF * Nfp);
+  const FastDiv by_np(Np), by_npm1(NpM1), by_nfp(Nfp), by_4nfp(4 * Nfp), by_nfnp(NF * Np);
     const int64_t e0 = tile * epb;
     const int ne = (int)min64(epb, K - e0);
     __syncthreads();
@@ -216,6 +269,10 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
       }
       sPen[2 * t] = cp;
       sPen[2 * t + 1] = cu;
+    }
+    if (sizeof(T) == 8 && L.stacks) {
+      const T* w = reinterpret_cast<const T*>(P.gtab + P.tab.o_wred);
+      for (int t = threadIdx.x; t < (N + 1) * (N + 2); t += blockDim.x) sbase[L.out + t] = __ldg(w + t);
     }
     // barycentric weights of J d/dx, J d/dy, J d/dz: g_a = (rxJ, sxJ, txJ, -sum) / 2, once
     // per element rather than per volume point
@@ -277,11 +334,19 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
         // 3d_wave.jl:45-54
         // the velocity flux 0.5 B (nx, ny, nz) is stored as the scalar 0.5 B; the lift
         // multiplies its result by the normal
+        if constexpr (sizeof(T) == 8) {  // the halves folded into n and cp (exact)
+          const T h = fma(T(0.5) * nz, d[3], fma(T(0.5) * ny, d[2], T(0.5) * nx * d[1]));
+          fl[0] = fma(T(0.5) * cp, d[0], -h);
+          fl[1] = fma(cu, h, -T(0.5) * d[0]);
+        } else {
         const T ndotdU = nx * d[1] + ny * d[2] + nz * d[3];
         const T A = cp * d[0] - ndotdU;
         const T B = cu * ndotdU - d[0];
         fl[0] = T(0.5) * A;
         fl[1] = T(0.5) * B;
+        }
+      } else if constexpr (sizeof(T) == 8) {
+        maxwell_flux<T>(d, nx, ny, nz, cp, cu, fl);
       } else {
         // 3d_maxwell.jl:52-63: 0.5 (fx nx + fy ny + fz nz)(du) + 0.5 du - 0.5 n (n.d)
         const T Hx = d[0], Hy = d[1], Hz = d[2], Ex = d[3], Ey = d[4], Ez = d[5];
@@ -296,13 +361,14 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
           fl[m] = T(0.5) * ax[m] * nx + T(0.5) * ay[m] * ny + T(0.5) * az[m] * nz +
                   T(0.5) * (cp * d[m]) - T(0.5) * (cu * nd[m]);
       }
-      T* fo = sFlux + ((size_t)(le * 4 + f) * NF) * Nfp + a;
+      T* fo = sFlux + ((size_t)(le * 4 + f) * (L.stacks ? NCH : NF)) * Nfp + a;
 #pragma unroll
       for (int ch = 0; ch < NCH; ++ch) fo[(size_t)ch * Nfp] = fl[ch];
     }
 
-    // ---- 3a. volume term at degree N-1 -------------------------------------------------
-    for (int it = threadIdx.x; it < ne * NpM1; it += blockDim.x) {
+    // ---- 3a. volume term at degree N-1 (from the last warp on: the flux above started with the
+    //          first, and a small tile keeps only some warps busy with each) ------------------
+    for (int it = blockDim.x - 1 - threadIdx.x; it < ne * NpM1; it += blockDim.x) {
       const int le = by_npm1.div(it), b = it - le * NpM1;
       const uint32_t c = st.node3m1[b];
       const int i = c & 0xff, j = (c >> 8) & 0xff, k = c >> 16;
@@ -329,7 +395,8 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
           const T p = F(0, a) - p3, u = F(1, a) - u3, v = F(2, a) - v3, ww = F(3, a) - w3;
-          w[0] += gx[a] * u + gy[a] * v + gz[a] * ww;
+          if constexpr (sizeof(T) == 8) w[0] = fma(gz[a], ww, fma(gy[a], v, fma(gx[a], u, w[0])));
+          else w[0] += gx[a] * u + gy[a] * v + gz[a] * ww;
           w[1] += gx[a] * p;
           w[2] += gy[a] * p;
           w[3] += gz[a] * p;
@@ -341,6 +408,10 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
         for (int a = 0; a < 3; ++a) {
           const T Hx = F(0, a) - Hx3, Hy = F(1, a) - Hy3, Hz = F(2, a) - Hz3;
           const T Ex = F(3, a) - Ex3, Ey = F(4, a) - Ey3, Ez = F(5, a) - Ez3;
+          if constexpr (sizeof(T) == 8) {
+            maxwell_curl<T>(w, gx[a], gy[a], gz[a], Hx, Hy, Hz, Ex, Ey, Ez);
+            continue;
+          }
           w[0] += -gy[a] * Ez + gz[a] * Ey;  // d/dt Hx = -dEz/dy + dEy/dz
           w[1] += gx[a] * Ez - gz[a] * Ex;   // d/dt Hy
           w[2] += -gx[a] * Ey + gy[a] * Ex;  // d/dt Hz
@@ -353,6 +424,96 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
       for (int m = 0; m < NW; ++m) sWork[((size_t)m * epb + le) * NpM1 + b] = w[m];
     }
     __syncthreads();
+    if (L.stacks) {
+      // ---- 3-5 with whole stacks: lift every face, then per coefficient the volume term, the
+      // four faces (t=-1 first as src/BernsteinLift.jl:202-205), 1/J and the update -----------
+      const int gs = Np | 1;
+      T* sG = sbase + L.stack;
+      lift_stacks<T>(N, ne * 4 * NCH, st.node2, sFlux, Nfp, sG, gs, sbase + L.out);
+      // one thread per coefficient and group of FG fields: the wave's all (its faces' scalar chain
+      // serves three), Maxwell's by twos, so that more warps share the pass (K = 2,058, N = 9:
+      // 256 -> 252 us per stage; the wave by twos 131 -> 140 us at N = 7, K = 4,374)
+      constexpr int FG = PHYS == BB_WAVE ? NF : PHYS == BB_MAXWELL ? 2 : 1;
+      const uint4* gtab4 = reinterpret_cast<const uint4*>(P.gtab + P.tab.o_gather);
+      const FastDiv by_gnp(NF / FG * Np);
+      for (int it = threadIdx.x; it < ne * (NF / FG) * Np; it += blockDim.x) {
+        const int le = by_gnp.div(it), rem = it - le * (NF / FG) * Np;
+        const int fg = by_np.div(rem), n = rem - fg * Np, f0 = fg * FG;
+        const uint4 ga = __ldg(gtab4 + n);
+        const uint32_t c = st.node3[n];
+        const int al[4] = {(int)(c & 0xff), (int)((c >> 8) & 0xff), (int)(c >> 16),
+                           N - (int)(c & 0xff) - (int)((c >> 8) & 0xff) - (int)(c >> 16)};
+        const int xb[4] = {(int)(ga.x & 0xffff), (int)(ga.x >> 16), (int)(ga.y & 0xffff),
+                           (int)(ga.y >> 16)};
+        const int pf[4] = {(int)(ga.z & 0xffff), (int)(ga.z >> 16), (int)(ga.w & 0xffff),
+                           (int)(ga.w >> 16)};
+        const size_t at = ((size_t)f0 * K + e0 + le) * Np + n, fs = (size_t)K * Np;
+        T res[FG];
+        if (P.mode != 0) {
+#pragma unroll
+          for (int m = 0; m < FG; ++m) res[m] = P.res[at + m * fs];
+        }
+        T acc[FG];
+#pragma unroll
+        for (int m = 0; m < FG; ++m) acc[m] = T(0);
+        if (NW == NF || f0 < NW) {  // fields past NW have no volume term
+          const T* wb = sWork + ((size_t)f0 * epb + le) * NpM1;
+          const size_t ws = (size_t)epb * NpM1;
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            if (al[b] == 0) continue;
+            const T v = small_int<T>(al[b]);
+#pragma unroll
+            for (int m = 0; m < FG; ++m) acc[m] = fma(v, wb[m * ws + xb[b]], acc[m]);
+          }
+          if (Phys<PHYS>::vol_sign < 0) {
+#pragma unroll
+            for (int m = 0; m < FG; ++m) acc[m] = -acc[m];
+          }
+        }
+        // the faces, t=-1 first as src/BernsteinLift.jl:202-205
+        const T* nc = sGeo + le * BB_GEO_STRIDE + 12;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int f = (q + 3) & 3;  // faces 3, 0, 1, 2
+          const T* g = sG + (size_t)((le * 4 + f) * NCH) * gs + pf[f];
+          if constexpr (PHYS == BB_WAVE) {
+            // field 0 takes the pressure chain, velocity component m - 1 the scalar chain times
+            // that component of the normal
+            const T s = g[gs];
+            acc[0] += g[0];
+#pragma unroll
+            for (int m = 1; m < NF; ++m) acc[m] = fma(nc[4 * (m - 1) + f], s, acc[m]);
+          } else {
+#pragma unroll
+            for (int m = 0; m < FG; ++m) acc[m] += g[(size_t)(f0 + m) * gs];
+          }
+        }
+        const T invJ = sGeo[le * BB_GEO_STRIDE + 9];
+        if (P.mode == 0) {
+#pragma unroll
+          for (int m = 0; m < FG; ++m) P.rhs[at + m * fs] = acc[m] * invJ;
+        } else {
+          const T dtJ = P.dt * invJ;
+#pragma unroll
+          for (int m = 0; m < FG; ++m) {
+            T* sq = sQ + ((size_t)(f0 + m) * epb + le) * Np + n;
+            T r;
+            if constexpr (sizeof(T) == 8) r = fma(dtJ, acc[m], P.rkA * res[m]);
+            else r = fma(P.rkA, res[m], P.dt * (acc[m] * invJ));
+            const T qn = fma(P.rkB, r, *sq);
+            P.res[at + m * fs] = r;
+            P.q[at + m * fs] = qn;
+            *sq = qn;
+          }
+        }
+      }
+      if (P.mode != 0 && P.trace_out) {
+        __syncthreads();
+        write_traces<T, NF>(P, st, sQ, sConn, e0, ne);
+      }
+      return;
+    }
     // ---- 3b. elevate back to degree N: out(alpha) = sign * sum_b alpha_b w(alpha - e_b) -
     for (int it = threadIdx.x; it < ne * Np; it += blockDim.x) {
       const int le = by_np.div(it), n = it - le * Np;
@@ -468,17 +629,7 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
       }
       if (P.trace_out) {
         __syncthreads();
-        for (int it = threadIdx.x; it < ne * 4 * NF * Nfp; it += blockDim.x) {
-          const int le = by_4nfnfp.div(it);
-          int rem = it - le * 4 * NF * Nfp;
-          const int f = by_nfnfp.div(rem);
-          rem -= f * NF * Nfp;
-          const int fld = by_nfp.div(rem), a = rem - fld * Nfp;
-          const int64_t nbr = (int64_t)((uint32_t)sConn[le * 4 + f] >> 5);
-          if (nbr >= e0 && nbr < e0 + ne) continue;  // neighbour inside the tile
-          P.trace_out[((size_t)(e0 + le) * 4 + f) * NF * Nfp + (size_t)fld * Nfp + a] =
-              sQ[((size_t)fld * epb + le) * Np + st.fvol[f * Nfp + a]];
-        }
+        write_traces<T, NF>(P, st, sQ, sConn, e0, ne);
       }
     }
 }
