@@ -193,7 +193,7 @@ def grad_(dr, ds, dt_, N: int, x, stream=None):
 
 
 def fused_apply_(dr, ds, dt_, lift_out, N: int, x, faces, stream=None):
-    """Dr x, Ds x, Dt x and L faces in one launch."""
+    """Dr x, Ds x, Dt x and L faces in one call (bb_fused_apply)."""
     N = _check_degree(N)
     K = _columns(x, np3(N), "x")
     if _columns(faces, 4 * np2(N), "faces") != K:

@@ -355,89 +355,64 @@ __global__ void __launch_bounds__(256) deriv_fact_kernel(DegTables tab,
 // -------------------------------------------------------------------------------------
 // lift kernels
 // -------------------------------------------------------------------------------------
+// Sum of the four face stacks at coefficient n of element le (t=-1 face first, then f1, f2, f3 as
+// src/BernsteinLift.jl:202-218); ga = the coefficient's entry of the gather table.
+template <class T>
+__device__ __forceinline__ T gather_faces(const T* sG, int gs, int le, uint4 ga) {
+  const T* g = sG + (size_t)le * 4 * gs;
+  return ((g[3 * gs + (ga.w >> 16)] + g[ga.z & 0xffff]) + g[gs + (ga.z >> 16)]) +
+         g[2 * gs + (ga.w & 0xffff)];
+}
+
+// Copies the double recursion's weights (lift_stacks) into shared memory.
+template <class T>
+__device__ __forceinline__ void load_wred(const DegTables& tab, const uint32_t* gtab, T* s) {
+  if (sizeof(T) != 8) return;
+  const T* w = reinterpret_cast<const T*>(gtab + tab.o_wred);
+  for (int t = threadIdx.x; t < (tab.N + 1) * (tab.N + 2); t += blockDim.x) s[t] = __ldg(w + t);
+}
+
+// Shared memory of lift_kernel in scalars: the weights, then per element the face inputs and
+// stacks.
+static size_t lift_scalars(const DegTables& t, int nfaces, int epb) {
+  return (size_t)(t.N + 1) * (t.N + 2) + (size_t)epb * nfaces * (t.Nfp + (t.Np | 1));
+}
+
 // Full lift (nfaces = 4) or single-face lift (nfaces = 1, face index 3 = the face written
-// directly, src/BernsteinLift.jl:139-164) of EPB element columns per block iteration.
+// directly, src/BernsteinLift.jl:139-164) of EPB element columns per block iteration: every face's
+// whole stack in shared memory (lift_stacks), then one pass sums the faces per coefficient. In
+// double the FP64 pipe bounds it (86 % of its rate at N = 7: 60,001 columns in 270 us, 417 with a
+// lift face by face that added every layer into the output, 4 (N+1) block barriers per tile).
 template <class T>
 __global__ void __launch_bounds__(256) lift_kernel(DegTables tab, const uint32_t* __restrict__ gtab,
                                                    int64_t K, int epb,
                                                    int nfaces, const T* __restrict__ x,
                                                    T* __restrict__ out) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const int N = tab.N, Np = tab.Np, Nfp = tab.Nfp;
-  const int S = np2(N + 1);
+  const int N = tab.N, Np = tab.Np, Nfp = tab.Nfp, gs = Np | 1;
   const int in_cols = nfaces * Nfp;
-  T* sin = reinterpret_cast<T*>(smem);
-  T* sout = sin + epb * in_cols;
-  T* bufA = sout + epb * Np;
-  T* bufB = bufA + epb * S;
+  T* wred = reinterpret_cast<T*>(smem);
+  T* sin = wred + (N + 1) * (N + 2);
+  T* sG = sin + (size_t)epb * in_cols;
   uint32_t* stab = reinterpret_cast<uint32_t*>(
-      smem + align16(sizeof(T) * ((size_t)epb * (in_cols + Np + 2 * S))));
+      smem + align16(sizeof(T) * ((N + 1) * (N + 2) + (size_t)epb * nfaces * (Nfp + gs))));
   const SmemTables st = load_tables(tab, gtab, stab);
+  load_wred(tab, gtab, wred);
+  const uint4* gather = reinterpret_cast<const uint4*>(gtab + tab.o_gather);
+  const FastDiv by_np(Np);
   const int64_t nblk = (K + epb - 1) / epb;
   for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
     const int64_t e0 = blk * epb;
     const int ne = (int)min64(epb, K - e0);
     __syncthreads();
     copy_g2s(sin, x + e0 * in_cols, ne * in_cols);
-    for (int t = threadIdx.x; t < ne * Np; t += blockDim.x) sout[t] = T(0);
     __syncthreads();
-    if (nfaces == 4) {
-      // face 4 (t = -1) first, then f1, f2, f3, as src/BernsteinLift.jl:202-218
-      for (int q = 0; q < 4; ++q) {
-        const int f = (q + 3) & 3;  // faces 3, 0, 1, 2
-        lift_face_accumulate<T>(N, f, ne, 1, st.node2, sin + f * Nfp, in_cols, 0, sout, Np, 0,
-                                bufA, bufB);
-      }
-    } else {
-      lift_face_accumulate<T>(N, 3, ne, 1, st.node2, sin, Nfp, 0, sout, Np, 0, bufA, bufB);
-    }
-    copy_s2g(out + e0 * Np, sout, ne * Np);
-  }
-}
-
-// Fused operator pass: Dr, Ds, Dt of the volume columns and the lift of the face columns
-// of the same EPB elements, one launch, each input read once.
-template <class T>
-__global__ void __launch_bounds__(256) fused_kernel(DegTables tab, const uint32_t* __restrict__ gtab,
-                                                    int64_t K, int epb,
-                                                    const T* __restrict__ x, const T* __restrict__ faces,
-                                                    T* __restrict__ dr, T* __restrict__ ds,
-                                                    T* __restrict__ dt, T* __restrict__ out) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int N = tab.N, Np = tab.Np, Nfp = tab.Nfp;
-  const int S = np2(N + 1);
-  const int in_cols = 4 * Nfp;
-  T* sx = reinterpret_cast<T*>(smem);
-  T* sin = sx + epb * Np;
-  T* sout = sin + epb * in_cols;
-  T* bufA = sout + epb * Np;
-  T* bufB = bufA + epb * S;
-  uint32_t* stab = reinterpret_cast<uint32_t*>(
-      smem + align16(sizeof(T) * ((size_t)epb * (Np + in_cols + Np + 2 * S))));
-  const SmemTables st = load_tables(tab, gtab, stab);
-  T* outs[3] = {dr, ds, dt};
-  const int64_t nblk = (K + epb - 1) / epb;
-  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
-    const int64_t e0 = blk * epb;
-    const int ne = (int)min64(epb, K - e0);
-    __syncthreads();
-    copy_g2s(sx, x + e0 * Np, ne * Np);
-    copy_g2s(sin, faces + e0 * in_cols, ne * in_cols);
-    for (int t = threadIdx.x; t < ne * Np; t += blockDim.x) sout[t] = T(0);
-    __syncthreads();
+    lift_stacks<T>(N, ne * nfaces, st.node2, sin, Nfp, sG, gs, wred);
     for (int it = threadIdx.x; it < ne * Np; it += blockDim.x) {
-      const int le = it / Np, row = it - le * Np;
-      const uint32_t c = st.node3[row];
-      const int i = c & 0xff, j = (c >> 8) & 0xff, k = c >> 16;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) outs[a][e0 * Np + it] = deriv_row<T>(a, N, sx + le * Np, i, j, k, row);
+      const int le = by_np.div(it), n = it - le * Np;
+      out[e0 * Np + it] = nfaces == 4 ? gather_faces(sG, gs, le, __ldg(gather + n))
+                                      : sG[(size_t)le * gs + n];
     }
-    for (int q = 0; q < 4; ++q) {
-      const int f = (q + 3) & 3;  // faces 3, 0, 1, 2
-      lift_face_accumulate<T>(N, f, ne, 1, st.node2, sin + f * Nfp, in_cols, 0, sout, Np, 0,
-                              bufA, bufB);
-    }
-    copy_s2g(out + e0 * Np, sout, ne * Np);
   }
 }
 
@@ -525,42 +500,21 @@ static int launch_lift(bb_ctx* ctx, const DegTables* t, int64_t K, int nfaces, c
     const int rc = bb_lift_fast(ctx, t, K, nfaces, x, out, st);
     if (rc >= 0) return rc;  // otherwise no specialised kernel for this degree
   }
-  const int S = np2(t->N + 1);
-  int epb = 8;
+  // the most elements (up to 16) within 54 KB, four blocks per SM (FP64, N = 7: 284 / 270 / 312 us
+  // for 60,001 columns with 36 / 54 / 110 KB)
+  int epb = 16;
   size_t smem = 0;
   for (; epb >= 1; epb /= 2) {
-    smem = align16(sizeof(T) * ((size_t)epb * (nfaces * t->Nfp + t->Np + 2 * S))) +
-           4 * (size_t)t->nwords;
-    if (smem <= 64 * 1024) break;
+    smem = align16(sizeof(T) * lift_scalars(*t, nfaces, epb)) + 4 * (size_t)t->nwords;
+    if (smem <= 54 * 1024 || epb == 1) break;
   }
-  if (epb < 1) return bb_fail(ctx, BB_ERR_ARG, "degree too large for lift tile");
+  if (smem > ctx->smem_optin) return bb_fail(ctx, BB_ERR_ARG, "degree too large for lift tile");
   BB_CUDA(ctx, cudaFuncSetAttribute(lift_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)smem));
   const int64_t nblk = (K + epb - 1) / epb;
-  lift_kernel<T><<<grid_for(ctx, nblk, 4), 256, smem, st>>>(*t, t->d_words, K, epb, nfaces,
+  lift_kernel<T><<<grid_for(ctx, nblk, 8), 256, smem, st>>>(*t, t->d_words, K, epb, nfaces,
                                                              (const T*)x, (T*)out);
   return bb_check_launch(ctx, "lift_kernel");
-}
-
-template <class T>
-static int launch_fused(bb_ctx* ctx, const DegTables* t, int64_t K, const void* x, const void* faces,
-                        void* dr, void* ds, void* dt, void* out, cudaStream_t st) {
-  const int S = np2(t->N + 1);
-  int epb = 8;
-  size_t smem = 0;
-  for (; epb >= 1; epb /= 2) {
-    smem = align16(sizeof(T) * ((size_t)epb * (2 * t->Np + 4 * t->Nfp + 2 * S))) +
-           4 * (size_t)t->nwords;
-    if (smem <= 64 * 1024) break;
-  }
-  if (epb < 1) return bb_fail(ctx, BB_ERR_ARG, "degree too large for fused tile");
-  BB_CUDA(ctx, cudaFuncSetAttribute(fused_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-  const int64_t nblk = (K + epb - 1) / epb;
-  fused_kernel<T><<<grid_for(ctx, nblk, 4), 256, smem, st>>>(*t, t->d_words, K, epb, (const T*)x,
-                                                              (const T*)faces, (T*)dr, (T*)ds,
-                                                              (T*)dt, (T*)out);
-  return bb_check_launch(ctx, "fused_kernel");
 }
 
 static int check_common(bb_ctx* ctx, int N, int64_t K, int dtype) {
@@ -666,12 +620,13 @@ extern "C" int bb_fused_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const vo
   const DegTables* t = bb_tables(ctx, N);
   if (!t) return bb_fail(ctx, BB_ERR_NOMEM, "table allocation failed");
   cudaStream_t st = (cudaStream_t)stream;
-  if (dtype == BB_F32 && N <= 15) {
-    // the gradient and lift calls back to back (degree-specialised kernels where they exist)
-    // move the same bytes faster than the one-launch table-driven pass
-    rc = launch_deriv<float>(ctx, t, K, 7, x, dr, ds, dt, st);
-    return rc ? rc : launch_lift<float>(ctx, t, K, 4, faces, lift, st);
-  }
-  return dtype == BB_F64 ? launch_fused<double>(ctx, t, K, x, faces, dr, ds, dt, lift, st)
-                         : launch_fused<float>(ctx, t, K, x, faces, dr, ds, dt, lift, st);
+  // The gradient and lift calls back to back. One launch that read each input once was slower in
+  // both precisions: FP64 is bound by its pipe (60,001 columns, N = 7: 505 us fused, 192 + 270
+  // apart), FP32 has specialised kernels, and above N = 15 (7,431 columns, N = 16) took 198 us
+  // against 60 + 117.
+  rc = dtype == BB_F64 ? launch_deriv<double>(ctx, t, K, 7, x, dr, ds, dt, st)
+                       : launch_deriv<float>(ctx, t, K, 7, x, dr, ds, dt, st);
+  if (rc) return rc;
+  return dtype == BB_F64 ? launch_lift<double>(ctx, t, K, 4, faces, lift, st)
+                         : launch_lift<float>(ctx, t, K, 4, faces, lift, st);
 }

@@ -97,10 +97,9 @@ int bb_elevation_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const void* x, 
 int bb_reduction_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const void* x, void* out,
                        void* stream);
 
-/* Fused operator pass: dr, ds, dt = D{r,s,t} x and lift = L faces. In FP32 with N <= 15
- * this is two launches, the gradient kernel and then the lift kernel, whose results equal
- * bb_grad_apply and bb_lift_apply bitwise; otherwise (FP64, N > 15) one launch of the
- * table-driven fused kernel. */
+/* Both operator passes: dr, ds, dt = D{r,s,t} x and lift = L faces, as two launches, the
+ * gradient kernel and then the lift kernel, whose results equal bb_grad_apply and
+ * bb_lift_apply bitwise. */
 int bb_fused_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const void* x,
                    const void* faces, void* dr, void* ds, void* dt, void* lift, void* stream);
 
