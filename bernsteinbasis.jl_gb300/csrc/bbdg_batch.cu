@@ -68,8 +68,7 @@ __global__ void __launch_bounds__(kBatchThreads, 3)
           s_phys = d.physics;
           s_begin = d.tile_begin;
           const int NF = physics_nf(d.physics);
-          sL = tile_layout_for(d.P.tab.N, NF, NF, sizeof(T), d.P.tab.nwords, d.P.epb,
-                               kBatchChainLiftBytes);
+          sL = tile_layout_for(d.P.tab.N, NF, NF, sizeof(T), d.P.tab.nwords, d.P.epb);
           s_prob = p;
           s_reload = 1;
         }
@@ -140,7 +139,7 @@ int batch_tile_default(int N, int nf, int dtype) {
   const int cands[4] = {6, 4, 2, 1};
   for (int e : cands) {
     const TileLayout L =
-        tile_layout_for(N, nf, nf, dtype_size(dtype), deg_table_words(N), e, kBatchChainLiftBytes);
+        tile_layout_for(N, nf, nf, dtype_size(dtype), deg_table_words(N), e);
     if (L.total <= 100 * 1024) return e;
   }
   return 1;
@@ -204,8 +203,7 @@ int build_desc(bb_batch* b) {
     d.physics = pr.physics;
     begin += (pr.K + b->epb[p] - 1) / b->epb[p];
     const int nf = physics_nf(pr.physics);
-    const TileLayout L = tile_layout_for(pr.N, nf, nf, sizeof(T), t->nwords, b->epb[p],
-                                         kBatchChainLiftBytes);
+    const TileLayout L = tile_layout_for(pr.N, nf, nf, sizeof(T), t->nwords, b->epb[p]);
     smem = std::max(smem, L.total);
   }
   b->ngeneric = (int)h.size();
@@ -450,7 +448,7 @@ extern "C" int bb_batch_set_tile(bb_batch* b, int physics, int N, int elems_per_
   const int nf = physics_nf(physics);
   if (!valid_degree(N) || nf == 0) return bb_fail(b->ctx, BB_ERR_ARG, "bad physics or degree");
   const TileLayout L = tile_layout_for(N, nf, nf, dtype_size(b->dtype), deg_table_words(N),
-                                       elems_per_block, kBatchChainLiftBytes);
+                                       elems_per_block);
   if (L.total > b->ctx->smem_optin)
     return bb_fail(b->ctx, BB_ERR_ARG, "tile of %d elements exceeds shared memory", elems_per_block);
   int hits = 0;

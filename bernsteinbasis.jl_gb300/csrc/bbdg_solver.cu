@@ -130,7 +130,7 @@ struct bb_solver {
 
 namespace {
 
-int solver_layout(bb_solver* s, int epb, size_t* smem_out, int* chain_out = nullptr) {
+int solver_layout(bb_solver* s, int epb, size_t* smem_out) {
   TileLayout L;
   if (s->physics == BB_WAVE)
     L = s->dtype == BB_F64 ? tile_layout<double, BB_WAVE>(*s->tab, epb)
@@ -145,26 +145,28 @@ int solver_layout(bb_solver* s, int epb, size_t* smem_out, int* chain_out = null
     L = s->dtype == BB_F64 ? tile_layout<double, BB_MAXWELL>(*s->tab, epb)
                            : tile_layout<float, BB_MAXWELL>(*s->tab, epb);
   *smem_out = L.total;
-  if (chain_out) *chain_out = L.chain;
   return L.total <= s->ctx->smem_optin ? BB_OK : BB_ERR_ARG;
 }
 
-// Default tile of the FP64 kernel with whole stacks (0: none fits). Its time is what the busiest
-// SM takes, tiles per SM times the elements of a tile plus a set-up worth about 150 coefficients
-// per tile (measured: wave N = 7, K = 4,374, 151 / 136 / 131 us per stage at 1 / 2 / 3 elements,
-// N = 3, K = 10,368, 171 / 109 / 85 / 70 / 68 at 1 / 2 / 3 / 6 / 8); tiles of several elements
-// count only where three blocks fit on an SM (Maxwell N = 7, K = 4,374: 301 / 305 / 360 at 1 / 2 / 3
-// elements, 4 / 2 / 1 blocks) and every SM gets two tiles (wave N = 7, K = 384: 22 / 26 us).
+// Default tile of the generic kernel with whole stacks (0: none fits). Its time is what the
+// busiest SM takes: tiles per SM times the elements of a tile plus a set-up per tile, worth about
+// 150 coefficients in FP64 and 60 per lift layer in FP32. Measured per stage at 1 / 2 / 3 / 4 / 6 /
+// 8 elements: FP64 wave N = 7, K = 4,374, 151 / 136 / 131 / 136 / 163 / 158 us, N = 3, K = 10,368,
+// 171 / 109 / 85 / 80 / 70 / 68; FP32 advection N = 9, K = 10,368, 149 / 94 / 83 / 71 / 64 / 56. Tiles of
+// several elements count only where three blocks fit on an SM (FP64 Maxwell N = 7, K = 4,374: 301 /
+// 305 / 360 at 4 / 2 / 1 blocks) and every SM gets two tiles (FP64 wave N = 7, K = 384: 22 / 26 us).
 int stack_tile(bb_solver* s) {
+  const bool f64 = s->dtype == BB_F64;
+  const double setup = (f64 ? 150.0 : 60.0 * (s->N + 1)) / (s->nf * s->tab->Np);
   int best = 0;
   double cost = 0.0;
-  for (int e : {1, 2, 3, 4, 6, 8}) {
-    const TileLayout L = tile_layout_for(s->N, s->nf, physics_nw(s->physics), sizeof(double),
-                                         s->tab->nwords, e);
+  for (int e : {1, 2, 3, 4, 6, 8, 12, 16, 24}) {
+    const TileLayout L = tile_layout_for(s->N, s->nf, physics_nw(s->physics),
+                                         dtype_size(s->dtype), s->tab->nwords, e);
     if (!L.stacks || L.total > s->ctx->smem_optin) continue;
     const int64_t tiles = (s->K + e - 1) / e, sms = s->ctx->num_sms;
     if (e > 1 && (3 * (L.total + 1024) > 228 * 1024 || tiles < 2 * sms)) continue;
-    const double c = (double)((tiles + sms - 1) / sms) * (e + 150.0 / (s->nf * s->tab->Np));
+    const double c = (double)((tiles + sms - 1) / sms) * (e + setup);
     if (!best || c <= cost) best = e, cost = c;
   }
   return best;
@@ -379,23 +381,9 @@ extern "C" int bb_solver_create(bb_ctx* ctx, int physics, int N, int64_t K, int 
   s->geo = geo;
   s->tau = tau;
   s->tab = t;
-  // default tile: the largest of 12, 6, 4, 2 elements whose tile runs the chain lift (FP32
-  // tiles that fit its shared-memory budget); else, in this order, 4, 2, 6, 12 or 1 elements
-  // within 100 KB; FP64 with whole stacks has its own rule
-  const int cands[2][5] = {{12, 6, 4, 2, 0}, {4, 2, 6, 12, 1}};
-  if (dtype == BB_F64) s->epb = stack_tile(s);
+  // default tile: stack_tile's; where no tile holds whole stacks, one element
+  s->epb = stack_tile(s);
   if (s->epb) solver_layout(s, s->epb, &s->smem);
-  for (int pass = 0; pass < 2 && !s->epb; ++pass)
-    for (int c : cands[pass]) {
-      size_t sm = 0;
-      int chain = 0;
-      if (c > 0 && solver_layout(s, c, &sm, &chain) == BB_OK && sm <= 100 * 1024 &&
-          (pass == 1 || chain)) {
-        s->epb = c;
-        s->smem = sm;
-        break;
-      }
-    }
   if (!s->epb) {
     size_t sm = 0;
     if (solver_layout(s, 1, &sm) != BB_OK) {
@@ -515,7 +503,7 @@ extern "C" int bb_stage_tile_bytes(int physics, int N, int dtype, int epb, int64
   const int nf = physics_nf(physics);
   const TileLayout L = tile_layout_for(N, nf, physics_nw(physics), dtype_size(dtype), nwords, epb);
   *bytes = (int64_t)L.total;
-  if (chain) *chain = L.chain;
+  if (chain) *chain = dtype == BB_F32 && L.stacks && L.total <= 100 * 1024;
   return BB_OK;
 }
 

@@ -72,29 +72,25 @@ struct StageParams {
   int* status;          // device error word
 };
 
-// Shared-memory layout of a tile (in units of T unless noted). chain != 0: the lift runs one
-// thread per (element, face, chain) with the face stacks in shared memory (FP32 tiles that fit
-// in kChainLiftBytes); chain == 0: the level-parallel lift with two ping-pong rows.
-// stacks != 0: every chain of the tile keeps its whole stack (lift_stacks), and the gather, the
-// volume term and the update are one pass (`out` and the weights of lift_stacks share an offset).
+// Shared-memory layout of a tile (in units of T unless noted). stacks != 0: every chain of the
+// tile keeps its whole lift stack (lift_stacks), and the gather, the volume term and the update
+// are one pass (`out` is then the table of lift_stacks' weights); stacks == 0, where those do not
+// fit: the lift goes face by face with two ping-pong rows and adds into `out`.
 struct TileLayout {
   size_t q, out, flux, work, stack, geo, pen, gh, conn_bytes, tab_bytes, total;
   int work_elems;
-  int chain, stacks;
+  int stacks;
 };
-constexpr size_t kChainLiftBytes = 100 * 1024;
-// The batched kernel uses the same rule, so that a tile timed on a single problem (how its
-// size is chosen per physics and degree) runs the same code inside the batch.
-constexpr size_t kBatchChainLiftBytes = kChainLiftBytes;
+constexpr size_t kStackBytes = 224 * 1024;
 
 // Lift chains per face for NF fields (Phys<PHYS>::NCH): the wave's velocity flux is a scalar
 // times the face normal, so its three components share one chain.
 __host__ __device__ inline int lift_chains(int NF) { return NF == 4 ? 2 : NF; }
 
 // Layout for degree N with Np/Nfp/NpM1 coefficients, NF fields, NW volume terms, scalars of
-// `tsize` bytes and `nwords` 32-bit table words.
-__host__ __device__ inline TileLayout tile_layout_with(int N, int NF, int NW, size_t tsize,
-                                                      int nwords, int epb, int chain) {
+// `tsize` bytes and `nwords` 32-bit table words: without whole stacks.
+__host__ __device__ inline TileLayout tile_layout_rows(int N, int NF, int NW, size_t tsize,
+                                                      int nwords, int epb) {
   TileLayout L;
   const size_t Np = np3(N), Nfp = np2(N), NpM1 = np3(N - 1), S = np2(N + 1);
   const size_t nch = (size_t)lift_chains(NF);
@@ -103,9 +99,7 @@ __host__ __device__ inline TileLayout tile_layout_with(int N, int NF, int NW, si
   L.out = off; off += (size_t)NF * epb * Np;
   L.flux = off; off += (size_t)epb * 4 * NF * Nfp;
   L.work = off;
-  const size_t wvol = (size_t)NW * epb * NpM1;
-  const size_t wlift = chain ? (size_t)epb * 4 * nch * (Np + (Nfp | 1))  // stacks + rows
-                             : 2 * (size_t)epb * nch * S;
+  const size_t wvol = (size_t)NW * epb * NpM1, wlift = 2 * (size_t)epb * nch * S;
   L.work_elems = (int)(wvol > wlift ? wvol : wlift);
   off += L.work_elems;
   L.geo = off; off += (size_t)epb * BB_GEO_STRIDE;
@@ -115,7 +109,6 @@ __host__ __device__ inline TileLayout tile_layout_with(int N, int NF, int NW, si
   L.conn_bytes = bytes; bytes += align16((size_t)epb * 4 * sizeof(int32_t));
   L.tab_bytes = bytes; bytes += (size_t)nwords * 4;
   L.total = align16(bytes);
-  L.chain = chain;
   L.stack = 0;
   L.stacks = 0;
   return L;
@@ -141,67 +134,18 @@ __host__ __device__ inline TileLayout tile_layout_stacks(int N, int NF, int NW, 
   L.conn_bytes = bytes; bytes += align16((size_t)epb * 4 * sizeof(int32_t));
   L.tab_bytes = bytes; bytes += (size_t)nwords * 4;
   L.total = align16(bytes);
-  L.chain = 0;
   L.stacks = 1;
   return L;
 }
 
-// FP32: the chain lift when its tile fits in `budget` bytes, else the level-parallel one.
-// FP64 always lifts level by level: the chain phase keeps one thread per (element, face, chain)
-// busy, too few to feed the FP64 pipe (wave N = 9, 2-element tiles: the pipe is 48 % busy with
-// chains against 80 % level-parallel, 2.38 against 1.65 ms per stage); with whole stacks
-// where they fit.
-constexpr size_t kStackBytes = 224 * 1024;
+// Whole stacks where they fit. They take the place of one thread per (element, face, chain), which
+// kept too few threads busy (FP32 scalar advection, N = 9, K = 10,368, 8 elements: 88 -> 56 us per
+// stage; N = 15, K = 3,072: 227 -> 72), and in FP64 of the face-by-face lift (Maxwell N = 7,
+// K = 4,374: 403 -> 301). Every form gives the same bits in FP32.
 __host__ __device__ inline TileLayout tile_layout_for(int N, int NF, int NW, size_t tsize,
-                                                     int nwords, int epb,
-                                                     size_t budget = kChainLiftBytes) {
-  if (tsize == 8) {
-    const TileLayout s = tile_layout_stacks(N, NF, NW, tsize, nwords, epb);
-    if (s.total <= kStackBytes) return s;
-  }
-  const TileLayout c = tile_layout_with(N, NF, NW, tsize, nwords, epb, 1);
-  return tsize == 4 && c.total <= budget ? c : tile_layout_with(N, NF, NW, tsize, nwords, epb, 0);
-}
-
-// One face lift chain for run-time N, one thread (src/BernsteinLift.jl:139-164):
-//   F_0 = L0 x (the 7-point stencil of (N+1)^2/2 R_{N+1} E_{N->N+1}), F_d = l_d E_d with
-//   E_d = R_{N-d+1} E_{d-1}, carried as F_d = -1/(d+1) [(i+1) F_{d-1}(i+1,j) +
-//   (j+1) F_{d-1}(i,j+1) + (N-d+1-i-j) F_{d-1}(i,j)] (l_d / l_{d-1} = -(N-d+1)/(d+1))
-// in place in ascending order on the thread's shared-memory row E (degree-N layout), each F_d
-// written to the face's stack g in volume order through the stack table fst (face f's
-// entries: layer d, then j, then i, i + j <= N - d). Per point the same arithmetic as
-// lift_face_accumulate, so both lifts give the same stacks.
-template <class T>
-__device__ void chain_lift_runtime(int N, const T* __restrict__ x, T* __restrict__ E,
-                                   T* __restrict__ g, const uint16_t* __restrict__ fst) {
-  int rb = 0;  // row offset of row j in the degree-N triangle
-  for (int j = 0; j <= N; ++j) {
-    const int rlen = N + 1 - j;
-    const int rbn = rb + rlen;          // row j + 1
-    const int rbp = rb - (rlen + 1);    // row j - 1 (used only when j > 0)
-    for (int i = 0; i < rlen; ++i) {
-      const T e = l0_point<T>(i, j, N - i - j, x, rb, rbn, rbp);
-      E[rb + i] = e;
-      g[fst[rb + i]] = e;  // layer 0: stack index = 2D index
-    }
-    rb = rbn;
-  }
-  int s = rb;  // == np2(N): first entry of layer 1
-  for (int d = 1; d <= N; ++d) {
-    const int n = N - d + 1;  // input degree of this reduction
-    const T cd = -inv_int<T>(d + 1);  // l_d / (l_{d-1} n)
-    int r = 0;
-    for (int j = 0; j < n; ++j) {
-      const int rn = r + (N + 1 - j);  // next row in the degree-N layout
-      for (int i = 0; i + j < n; ++i) {
-        // in place, ascending: (i+1, j) and (i, j+1) are still degree-n values
-        const T v = reduce_point<T>(i, j, n, E[r + i + 1], E[rn + i], E[r + i], cd);
-        E[r + i] = v;
-        g[fst[s++]] = v;
-      }
-      r = rn;
-    }
-  }
+                                                     int nwords, int epb) {
+  const TileLayout s = tile_layout_stacks(N, NF, NW, tsize, nwords, epb);
+  return s.total <= kStackBytes ? s : tile_layout_rows(N, NF, NW, tsize, nwords, epb);
 }
 
 template <class T, int PHYS>
@@ -230,7 +174,7 @@ __device__ void write_traces(const StageParams<T>& P, const SmemTables& st, cons
 
 // One tile of the generic stage (all threads of the block call it). The degree tables are in
 // shared memory (st); the layout L matches P's degree, physics and tile.
-template <class T, int PHYS, bool CHAIN_LIFT = true>
+template <class T, int PHYS>
 __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
                                    const SmemTables& st, int64_t tile) {
   constexpr int NF = Phys<PHYS>::NF, NW = Phys<PHYS>::NW, NCH = Phys<PHYS>::NCH;
@@ -247,7 +191,7 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
   const int N = P.tab.N, Np = P.tab.Np, NpM1 = P.tab.NpM1, Nfp = P.tab.Nfp;
   const int64_t K = P.K;
   const int epb = P.epb;
-  const FastDiv by_np(Np), by_npm1(NpM1), by_nfp(Nfp), by_4nfp(4 * Nfp), by_nfnp(NF * Np);
+  const FastDiv by_np(Np), by_npm1(NpM1), by_nfp(Nfp), by_4nfp(4 * Nfp);
     const int64_t e0 = tile * epb;
     const int ne = (int)min64(epb, K - e0);
     __syncthreads();
@@ -553,43 +497,7 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
     __syncthreads();
 
     // ---- 4. lift of the face fluxes, face t=-1 first as src/BernsteinLift.jl:202-205 ----
-    if (CHAIN_LIFT && L.chain) {
-      // one thread per (element, face, chain); stacks land in volume order
-      const int nchain = ne * 4 * NCH;
-      const int rs = Nfp | 1;
-      T* sStack = sWork;                                // [epb*4*NCH][Np]
-      T* sRow = sWork + (size_t)epb * 4 * NCH * Np;     // [epb*4*NCH][rs]
-      for (int c = threadIdx.x; c < nchain; c += blockDim.x) {
-        const int ef = c / NCH, ch = c - ef * NCH;      // c = (le*4 + f)*NCH + ch
-        chain_lift_runtime<T>(N, sFlux + ((size_t)ef * NF + ch) * Nfp, sRow + (size_t)c * rs,
-                              sStack + (size_t)c * Np, st.fstack + (size_t)(ef & 3) * Np);
-      }
-      __syncthreads();
-      // faces in the order 3, 0, 1, 2 (as lift_face_accumulate, so that both lifts agree)
-      for (int it = threadIdx.x; it < ne * NF * Np; it += blockDim.x) {
-        const int le = by_nfnp.div(it), rem = it - le * NF * Np;
-        const int fld = by_np.div(rem), n = rem - fld * Np;
-        T* o = sOut + ((size_t)fld * epb + le) * Np + n;
-        T acc = *o;
-        if (PHYS == BB_WAVE && fld > 0) {
-          // velocity component fld - 1: the scalar chain times that normal component
-          const T* g = sStack + ((size_t)le * 4 * NCH + 1) * Np + n;  // face f at + f*NCH*Np
-          const T* nc = sGeo + le * BB_GEO_STRIDE + 12 + 4 * (fld - 1);
-          acc = fma(nc[3], g[(size_t)3 * NCH * Np], acc);
-          acc = fma(nc[0], g[0], acc);
-          acc = fma(nc[1], g[(size_t)1 * NCH * Np], acc);
-          acc = fma(nc[2], g[(size_t)2 * NCH * Np], acc);
-        } else {
-          const T* g = sStack + ((size_t)le * 4 * NCH + fld) * Np + n;
-          acc += g[(size_t)3 * NCH * Np];
-          acc += g[0];
-          acc += g[(size_t)1 * NCH * Np];
-          acc += g[(size_t)2 * NCH * Np];
-        }
-        *o = acc;
-      }
-      __syncthreads();
-    } else {
+    {
       const int S = np2(N + 1);
       T* bufA = sWork;
       T* bufB = sWork + (size_t)epb * NCH * S;

@@ -118,8 +118,8 @@ int bb_solver_destroy(bb_solver* s);
  * registers, tiles copied ahead); their last tile may be partial, so any K will do. */
 int bb_solver_set_tile(bb_solver* s, int elems_per_block, int threads);
 int bb_solver_get_tile(const bb_solver* s, int* elems_per_block, int* threads);
-/* Shared memory of one generic-kernel tile of epb elements (and whether it runs the
- * chain-per-thread lift), for tile choosers. */
+/* Shared memory of one generic-kernel tile of epb elements (and, in *chain, whether it is an
+ * FP32 tile within 100 KB that keeps every chain's whole lift stack), for tile choosers. */
 int bb_stage_tile_bytes(int physics, int N, int dtype, int epb, int64_t* bytes, int* chain);
 /* The idx-th compiled degree-specialised FP32 stage-kernel variant (idx = 0, 1, ...): its
  * degree, physics, elements per block and threads per block, for tile choosers; BB_ERR_ARG
