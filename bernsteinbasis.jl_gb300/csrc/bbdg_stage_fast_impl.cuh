@@ -507,6 +507,11 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
         const float ndotdU = nx * d[1] + ny * d[2] + nz * d[3];
         xin[0] = 0.5f * (cp * d[0] - ndotdU);    // p flux
         xin[NFP] = 0.5f * (cu * ndotdU - d[0]);  // (u,v,w) flux / n
+      } else if constexpr (!generic_order(N)) {
+        float fl[6];
+        maxwell_flux<float>(d, nx, ny, nz, cp, cu, fl);
+#pragma unroll
+        for (int m = 0; m < 6; ++m) xin[m * NFP] = fl[m];
       } else {
         const float Hx = d[0], Hy = d[1], Hz = d[2], Ex = d[3], Ey = d[4], Ez = d[5];
         const float ndH = nx * Hx + ny * Hy + nz * Hz;
@@ -624,6 +629,10 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
             const float Ex = q0[3 * EPB * NP + idx[a]] - x3[3],
                         Ey = q0[4 * EPB * NP + idx[a]] - x3[4],
                         Ez = q0[5 * EPB * NP + idx[a]] - x3[5];
+            if constexpr (!generic_order(N)) {
+              maxwell_curl<float>(w, gx[a], gy[a], gz[a], Hx, Hy, Hz, Ex, Ey, Ez);
+              continue;
+            }
             w[0] += -gy[a] * Ez + gz[a] * Ey;
             w[1] += gx[a] * Ez - gz[a] * Ex;
             w[2] += -gx[a] * Ey + gy[a] * Ex;
