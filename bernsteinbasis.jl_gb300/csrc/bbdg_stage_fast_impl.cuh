@@ -60,17 +60,20 @@ struct FPhys<BB_MAXWELL> {
   static constexpr int NF = 6, NCH = 6, NW = 6;
 };
 
-// From degree 12 on the arithmetic is the generic kernel's, operation by operation, so that a
-// state does not depend on which kernel advanced it: there one step amplifies a difference in
-// the last bit to 1e-5 of the state (degree 15), where it stays below 1e-7 up to degree 11. The
-// extra product per stack entry costs 3 % (wave N = 15).
-__host__ __device__ constexpr bool generic_order(int N) { return N >= 12; }
-// a * b; in generic order a rounded product: where a following weight is the constant 1 the
-// compiler would otherwise turn fma(1, x, a * b) into fma(a, b, x).
-template <int N>
-__device__ __forceinline__ float prod(float a, float b) {
-  return generic_order(N) ? __fmul_rn(a, b) : a * b;
+// Degrees whose lifts the element warps do, a warp per pair of chains and a lane per entry
+// (lift_pair_warp), instead of the chain warps with a chain per lane (lift_chain): fewer
+// instructions in all, until a chain outgrows a thread's registers and 16 or 24 of them make
+// 4,600 instructions in a row. Per stage, chain / warp: wave N = 15, K = 6,000, 235 / 145 us; N = 12,
+// K = 10,368, 154 / 136; N = 11, K = 16,464, 181 / 172; N = 10, 126 / 142; Maxwell N = 15, K = 3,072,
+// 227 / 160; N = 13, K = 6,000, 317 / 233; N = 11, K = 10,368, 197 / 261.
+template <int PHYS>
+__host__ __device__ constexpr bool warp_lift(int N) {
+  return PHYS == BB_MAXWELL ? N >= 12 : N >= 11;
 }
+// From degree 12 on the arithmetic is the generic kernel's, operation by operation, so that a
+// state does not depend on which kernel advanced it: there one step amplifies a difference in the
+// last bit to 1e-5 of the state (degree 15), where it stays below 1e-7 up to degree 11.
+__host__ __device__ constexpr bool generic_order(int N) { return N >= 12; }
 
 template <int N, int PHYS, int EPB, int TPE>
 struct FastLayout {
@@ -86,7 +89,9 @@ struct FastLayout {
   // stack entry q of chain ch at ((e4 * NPS + stack_slot<N>(q)) * NCH + ch). NPS = 1 mod 16
   // puts the same slot of the 32 chains of a warp (consecutive e4 and ch) in 32 different
   // banks for NCH = 2 and 6; the slots spread the gather's reads over the banks.
-  static constexpr int NSLOT = StackSlots<N>::span > NP ? StackSlots<N>::span : NP;
+  // (in volume order where a warp lifts: its stores are consecutive)
+  static constexpr int NSLOT =
+      !warp_lift<PHYS>(N) && StackSlots<N>::span > NP ? StackSlots<N>::span : NP;
   static constexpr int NPS = (NSLOT + 14) / 16 * 16 + 1;
   // w(beta) rows: NPM1 entries, then NZ zero entries from Z0 (a multiple of 8) on, one per bank
   // group of the gather's vector loads (16-byte entries: 8 lanes per phase, 8 groups; 24-byte
@@ -111,7 +116,8 @@ struct FastLayout {
   static constexpr int FPERM_B = FVOL_B + ((4 * NFP * 2 + 3) / 4 * 4);  // [6][NFP] u16
   static constexpr int FNB_B = FPERM_B + ((6 * NFP * 2 + 3) / 4 * 4);  // [4][6][NFP] u16
   static constexpr int TF_B = (FNB_B + 24 * NFP * 2 + 15) / 16 * 16;   // [NP] u32 face nodes
-  static constexpr int BAR_B = (TF_B + NP * 4 + 15) / 16 * 16;         // 4 mbarriers
+  static constexpr int DEC_B = (TF_B + NP * 4 + 15) / 16 * 16;  // [NP] u16, lift_pair_warp only
+  static constexpr int BAR_B = (DEC_B + (warp_lift<PHYS>(N) ? NP * 2 : 0) + 15) / 16 * 16;  // 4 mbarriers
   static constexpr int TABLES = BAR_B - GA_B;  // the constant tables, one image (fast_image)
   static constexpr int BYTES = BAR_B + 32;
   // element groups for the named-barrier hand-offs between the chain warps and the element
@@ -215,25 +221,16 @@ __device__ __forceinline__ void mbar_arrive_async(uint64_t* bar) {
 template <int N, int NCH>
 __device__ __forceinline__ void lift_chain(const float* x, float* g) {
   constexpr int NFP = (N + 1) * (N + 2) / 2;
-  // The inputs enter row by row: the stencil of row j reads rows j - 1, j and j + 1, so from
-  // N = 12 on, where two full triangles would not fit in the registers, only three rows of X are
-  // live beside E (N = 15: 136 + 45 values).
   float X[NFP];
-  constexpr int AHEAD = N >= 12 ? 1 : N;  // rows of X loaded ahead of the stencil
 #pragma unroll
-  for (int m = 0; m < c_tri(N, AHEAD < N ? AHEAD : N + 1); ++m) X[m] = x[m];
+  for (int m = 0; m < NFP; ++m) X[m] = x[m];
   float E[NFP];
 #pragma unroll
   for (int j = 0; j <= N; ++j) {
-    if (AHEAD < N && j + 1 <= N) {
-#pragma unroll
-      for (int i = 0; i + j + 1 <= N; ++i) X[c_ij(N, i, j + 1)] = x[c_ij(N, i, j + 1)];
-    }
 #pragma unroll
     for (int i = 0; i + j <= N; ++i) {
       const int k = N - i - j;
-      float v = prod<N>(float((i + 1) * (i + 1) + (j + 1) * (j + 1) + (k + 1) * (k + 1)),
-                        X[c_ij(N, i, j)]);
+      float v = float((i + 1) * (i + 1) + (j + 1) * (j + 1) + (k + 1) * (k + 1)) * X[c_ij(N, i, j)];
       if (j > 0) v = fmaf(float((i + 1) * j), X[c_ij(N, i + 1, j - 1)], v);
       if (k > 0) v = fmaf(float((i + 1) * k), X[c_ij(N, i + 1, j)], v);
       if (i > 0) v = fmaf(float((j + 1) * i), X[c_ij(N, i - 1, j + 1)], v);
@@ -255,18 +252,82 @@ __device__ __forceinline__ void lift_chain(const float* x, float* g) {
       for (int i = 0; i + j < n; ++i) {
         // reduction_multiply! (src/BernsteinLift.jl:81-85) times l_d / l_{d-1}, in place in
         // ascending order
-        const float v =
-            generic_order(N)
-                ? fmaf(float(i + 1), E[c_ij(N, i + 1, j)],
-                       fmaf(float(j + 1), E[c_ij(N, i, j + 1)],
-                            prod<N>(float(n - i - j), E[c_ij(N, i, j)]))) * inv
-                : float(i + 1) * inv * E[c_ij(N, i + 1, j)] +
-                      (float(j + 1) * inv * E[c_ij(N, i, j + 1)] +
-                       float(n - i - j) * inv * E[c_ij(N, i, j)]);
+        const float v = float(i + 1) * inv * E[c_ij(N, i + 1, j)] +
+                        (float(j + 1) * inv * E[c_ij(N, i, j + 1)] +
+                         float(n - i - j) * inv * E[c_ij(N, i, j)]);
         E[c_ij(N, i, j)] = v;
         g[stack_slot<N>(c_ijk(N, i, j, d)) * NCH] = v;
       }
     }
+  }
+}
+
+// The lifts of two chains of a face by one warp, level-parallel (src/BernsteinLift.jl:139-164): xa,
+// xb = their inputs, g = the face's stack at the pair, entries NCH floats apart in volume order.
+// dec = (i | j << 8) of entry m of a degree-n triangle at np3(n-1) + m. Layer d is formed from layer
+// d-1 where it lies in the stack; the neighbours of entry m of a degree-n layer are m + 1 and
+// m + n + 1 - j. Two shared reads or writes of 8 bytes serve both chains.
+template <int N, int NCH>
+__device__ __forceinline__ void lift_pair_warp(const float* xa, const float* xb, float* g,
+                                               const uint16_t* dec, int lane) {
+  constexpr int NFP = (N + 1) * (N + 2) / 2;
+  {
+    const uint16_t* dc = dec + np3(N - 1);
+    for (int m = lane; m < NFP; m += 32) {
+      const int i = dc[m] & 0xff, j = dc[m] >> 8, k = N - i - j;
+      const int up = m + N + 1 - j, dn = m - (N + 2 - j);  // (i, j+1), (i, j-1)
+      const float w0 = float((i + 1) * (i + 1) + (j + 1) * (j + 1) + (k + 1) * (k + 1));
+      float a = __fmul_rn(w0, xa[m]), b = __fmul_rn(w0, xb[m]);
+      auto add = [&](int w, int at) {
+        a = fmaf(float(w), xa[at], a);
+        b = fmaf(float(w), xb[at], b);
+      };
+      if (j > 0) add((i + 1) * j, dn + 1);
+      if (k > 0) add((i + 1) * k, m + 1);
+      if (i > 0) add((j + 1) * i, up - 1);
+      if (k > 0) add((j + 1) * k, up);
+      if (i > 0) add((k + 1) * i, m - 1);
+      if (j > 0) add((k + 1) * j, dn);
+      *reinterpret_cast<float2*>(g + m * NCH) = make_float2(0.5f * a, 0.5f * b);
+    }
+  }
+  __syncwarp();
+  float* src = g;
+#pragma unroll
+  for (int n = N; n >= 1; --n) {  // degree n -> n - 1, layer N + 1 - n
+    const float inv = -1.0f / float(N + 2 - n);
+    const int cnt = n * (n + 1) / 2;
+    float* dst = src + (n + 1) * (n + 2) / 2 * NCH;
+    const uint16_t* dc = dec + (n - 1) * n * (n + 1) / 6;
+    // every load of the layer before its first store, which the compiler must keep behind them
+    constexpr int R = (NFP + 31) / 32;
+    float2 e0[R], e1[R], e2[R];
+    int ij[R];
+#pragma unroll
+    for (int r = 0; r * 32 < cnt; ++r) {
+      const int m = lane + 32 * r;
+      if (m < cnt) {
+        ij[r] = dc[m];
+        const int j = ij[r] >> 8;
+        const float* x = src + (m + j) * NCH;  // row j of the degree-n triangle starts j later
+        e0[r] = *reinterpret_cast<const float2*>(x);
+        e1[r] = *reinterpret_cast<const float2*>(x + NCH);
+        e2[r] = *reinterpret_cast<const float2*>(x + (n + 1 - j) * NCH);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r * 32 < cnt; ++r) {
+      const int m = lane + 32 * r;
+      if (m < cnt) {
+        const int i = ij[r] & 0xff, j = ij[r] >> 8;
+        const float wi = float(i + 1), wj = float(j + 1), wk = float(n - i - j);
+        *reinterpret_cast<float2*>(dst + m * NCH) =
+            make_float2(fmaf(wi, e1[r].x, fmaf(wj, e2[r].x, __fmul_rn(wk, e0[r].x))) * inv,
+                        fmaf(wi, e1[r].y, fmaf(wj, e2[r].y, __fmul_rn(wk, e0[r].y))) * inv);
+      }
+    }
+    src = dst;
+    __syncwarp();
   }
 }
 
@@ -301,6 +362,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   uint16_t* sFnb = reinterpret_cast<uint16_t*>(smem + L::FNB_B);
   // per coefficient: its node index on faces f0..f3 (one byte each, 0xff = not on the face)
   uint32_t* sTF = reinterpret_cast<uint32_t*>(smem + L::TF_B);
+  const uint16_t* sDec = reinterpret_cast<const uint16_t*>(smem + L::DEC_B);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_B);  // [0],[1] q slots, [2] res,
                                                                  // [3] tables
   __shared__ int s_fail;
@@ -575,12 +637,21 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
         }
       }
       const int c = tid - NTE;
-      if (!*vfail && c < NCHAIN)  // a partial tile's spare chains lift stale inputs, unused
-        lift_chain<N, NCH>(sX + (s * NCHAIN + c) * NFP, sG + (c / NCH) * NPS * NCH + c % NCH);
+      if constexpr (!warp_lift<PHYS>(N)) {
+        if (!*vfail && c < NCHAIN)  // a partial tile's spare chains lift stale inputs, unused
+          lift_chain<N, NCH>(sX + (s * NCHAIN + c) * NFP, sG + (c / NCH) * NPS * NCH + c % NCH);
+      }
       for (int g = 0; g < NG; ++g) nbar_arrive(1 + g, GCOUNT);
     } else if (it > 0 && (nbar_sync(1 + NG + grp, GCOUNT), *vfail)) {
       // a wait ran out: keep to the barrier sequence, skip the work
     } else {
+      if constexpr (warp_lift<PHYS>(N)) {  // this element's lifts, one pair of chains per warp
+        for (int q = u >> 5; q < 2 * NCH; q += TPE / 32) {
+          const int f = q / (NCH / 2), ch = 2 * (q - f * (NCH / 2));
+          const float* xa = sX + (s * NCHAIN + (le * 4 + f) * NCH + ch) * NFP;
+          lift_pair_warp<N, NCH>(xa, xa + NFP, sG + (le * 4 + f) * NPS * NCH + ch, sDec, u & 31);
+        }
+      }
       // the tile after next: its outside-tile neighbour traces (one contiguous NF x Nfp block
       // per face) are pulled into L2 now, a whole tile ahead of its flux phase
       const int tpre = tnext + step;
@@ -959,8 +1030,9 @@ std::vector<uint8_t> fast_image() {
       mb[b] = (uint32_t)(L::Z0 + zs);
     }
     // stack slots of this coefficient on faces f0 (i,k,j), f1 (j,k,l), f2 (j,k,i), f3 (i,j,k)
-    const uint32_t p0 = stack_slot<N>(ijk3(N, i, k, j)), p1 = stack_slot<N>(ijk3(N, j, k, l));
-    const uint32_t p2 = stack_slot<N>(ijk3(N, j, k, i)), p3 = stack_slot<N>(t);
+    auto slot = [](int q) { return (uint32_t)(warp_lift<PHYS>(N) ? q : stack_slot<N>(q)); };
+    const uint32_t p0 = slot(ijk3(N, i, k, j)), p1 = slot(ijk3(N, j, k, l));
+    const uint32_t p2 = slot(ijk3(N, j, k, i)), p3 = slot(t);
     // 10-bit fields: [0] w indices of alpha - e_b for b = 0..2, [1] stack slots on f0..f2, [3]
     // stack slot on f3 and the w index for b = 3; [2] alpha's barycentric indices, one byte each
     ga[4 * t] = mb[0] | (mb[1] << 10) | (mb[2] << 20);
@@ -990,6 +1062,12 @@ std::vector<uint8_t> fast_image() {
         fperm[o * NFP + q] = (uint16_t)ij2(N, wn[0], wn[1]);
       }
     }
+  if (warp_lift<PHYS>(N)) {
+    uint16_t* dec = reinterpret_cast<uint16_t*>(at(L::DEC_B));
+    for (int n = 0, q = 0; n <= N; ++n)
+      for (int b = 0; b <= n; ++b)
+        for (int a = 0; a <= n - b; ++a, ++q) dec[q] = (uint16_t)(a | (b << 8));
+  }
   for (int f = 0; f < 4; ++f)
     for (int o = 0; o < 6; ++o)
       for (int q = 0; q < NFP; ++q) fnb[(f * 6 + o) * NFP + q] = fvol[f * NFP + fperm[o * NFP + q]];

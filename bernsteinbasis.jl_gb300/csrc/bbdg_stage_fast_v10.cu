@@ -3,7 +3,10 @@
 #include "bbdg_stage_fast_impl.cuh"
 
 template struct bbfast::FastKernel<10, BB_WAVE, 2, 64>;
+template struct bbfast::FastKernel<10, BB_MAXWELL, 2, 192>;
 template struct bbfast::FastKernel<10, BB_MAXWELL, 2, 96>;
 template struct bbfast::FastKernel<10, BB_MAXWELL, 2, 64>;
+template struct bbfast::FastKernel<11, BB_WAVE, 2, 128>;
 template struct bbfast::FastKernel<11, BB_WAVE, 2, 96>;
+template struct bbfast::FastKernel<11, BB_MAXWELL, 2, 192>;
 template struct bbfast::FastKernel<11, BB_MAXWELL, 2, 96>;

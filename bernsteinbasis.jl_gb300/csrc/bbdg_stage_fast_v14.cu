@@ -2,7 +2,7 @@
 // degrees so that the variants compile in parallel).
 #include "bbdg_stage_fast_impl.cuh"
 
-template struct bbfast::FastKernel<14, BB_WAVE, 2, 160>;
-template struct bbfast::FastKernel<14, BB_MAXWELL, 1, 256>;
-template struct bbfast::FastKernel<15, BB_WAVE, 2, 160>;
-template struct bbfast::FastKernel<15, BB_MAXWELL, 1, 256>;
+template struct bbfast::FastKernel<14, BB_WAVE, 2, 256>;
+template struct bbfast::FastKernel<14, BB_MAXWELL, 1, 384>;
+template struct bbfast::FastKernel<15, BB_WAVE, 2, 256>;
+template struct bbfast::FastKernel<15, BB_MAXWELL, 1, 448>;

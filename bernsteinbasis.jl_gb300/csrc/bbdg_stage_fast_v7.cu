@@ -6,5 +6,6 @@ template struct bbfast::FastKernel<7, BB_WAVE, 4, 32>;
 template struct bbfast::FastKernel<7, BB_WAVE, 4, 64>;
 template struct bbfast::FastKernel<7, BB_MAXWELL, 2, 64>;
 template struct bbfast::FastKernel<8, BB_WAVE, 4, 64>;
+template struct bbfast::FastKernel<8, BB_MAXWELL, 4, 64>;
 template struct bbfast::FastKernel<8, BB_MAXWELL, 4, 32>;
 template struct bbfast::FastKernel<7, BB_WAVE, 2, 64>;

@@ -5,5 +5,6 @@
 template struct bbfast::FastKernel<9, BB_WAVE, 4, 64>;
 template struct bbfast::FastKernel<9, BB_WAVE, 4, 32>;
 template struct bbfast::FastKernel<9, BB_WAVE, 2, 64>;
+template struct bbfast::FastKernel<9, BB_MAXWELL, 2, 128>;
 template struct bbfast::FastKernel<9, BB_MAXWELL, 2, 64>;
 template struct bbfast::FastKernel<9, BB_MAXWELL, 2, 96>;
