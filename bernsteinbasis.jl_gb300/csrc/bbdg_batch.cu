@@ -89,23 +89,6 @@ __global__ void __launch_bounds__(kBatchThreads, 3)
   }
 }
 
-template <class T, int NF>
-__global__ void batch_extract_kernel(DegTables tab, const uint32_t* __restrict__ gtab, int64_t K,
-                                     const T* __restrict__ q, T* __restrict__ tr) {
-  const int Np = tab.Np, Nfp = tab.Nfp;
-  const uint16_t* fvol = reinterpret_cast<const uint16_t*>(gtab + tab.o_fvol);
-  const int64_t total = K * 4 * NF * Nfp;
-  for (int64_t it = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; it < total;
-       it += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = it / (4 * NF * Nfp);
-    int rem = (int)(it - e * 4 * NF * Nfp);
-    const int f = rem / (NF * Nfp);
-    rem -= f * NF * Nfp;
-    const int fld = rem / Nfp, a = rem - fld * Nfp;
-    tr[it] = q[((size_t)fld * K + e) * Np + fvol[f * Nfp + a]];
-  }
-}
-
 }  // namespace
 
 struct bb_batch {
@@ -300,18 +283,8 @@ int batch_extract(bb_batch* b, cudaStream_t st) {
     const bb_batch_problem& pr = b->probs[p];
     const DegTables& t = *b->tabs[p];
     const int nf = physics_nf(pr.physics);
-    int64_t grid = (pr.K * 4 * nf * t.Nfp + 255) / 256;
-    grid = std::min<int64_t>(std::max<int64_t>(grid, 1), (int64_t)b->ctx->num_sms * 8);
-    if (nf == 4)
-      batch_extract_kernel<T, 4><<<(int)grid, 256, 0, st>>>(t, t.d_words, pr.K, (const T*)pr.q,
-                                                            (T*)b->trace[2 * p]);
-    else if (nf == 1)
-      batch_extract_kernel<T, 1><<<(int)grid, 256, 0, st>>>(t, t.d_words, pr.K, (const T*)pr.q,
-                                                            (T*)b->trace[2 * p]);
-    else
-      batch_extract_kernel<T, 6><<<(int)grid, 256, 0, st>>>(t, t.d_words, pr.K, (const T*)pr.q,
-                                                            (T*)b->trace[2 * p]);
-    int rc = bb_check_launch(b->ctx, "batch_extract_kernel");
+    extract_traces<T>(t, nf, pr.K, pr.q, b->trace[2 * p], 0, pr.K, b->ctx->num_sms, st);
+    int rc = bb_check_launch(b->ctx, "extract_traces_kernel");
     if (rc) return rc;
   }
   return BB_OK;

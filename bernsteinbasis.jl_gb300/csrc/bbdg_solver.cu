@@ -27,33 +27,6 @@ __global__ void __launch_bounds__(2 * kThreads, 2) stage_kernel(StageParams<T> P
     generic_stage_tile<T, PHYS>(P, L, st, tile);
 }
 
-// Writes every face trace (all faces) of elements [e_begin, e_end) of q into the trace buffer.
-// An element's 4 NF Nfp trace entries are contiguous in the buffer; each block first decodes
-// entry i into (field, volume node) once (shared table), then copies element after element:
-// one table read, one gather from the element's field rows, one coalesced store per entry.
-template <class T, int NF>
-__global__ void extract_traces_kernel(DegTables tab, const uint32_t* __restrict__ gtab,
-                                      int64_t K, const T* __restrict__ q, T* __restrict__ tr,
-                                      int64_t e_begin, int64_t e_end) {
-  extern __shared__ uint32_t s_src[];  // entry i: field << 16 | volume node
-  const int Np = tab.Np, Nfp = tab.Nfp, W = 4 * NF * Nfp;
-  const uint16_t* fvol = reinterpret_cast<const uint16_t*>(gtab + tab.o_fvol);
-  for (int i = threadIdx.x; i < W; i += blockDim.x) {
-    const int f = i / (NF * Nfp), rem = i - f * NF * Nfp, fld = rem / Nfp, a = rem - fld * Nfp;
-    s_src[i] = ((uint32_t)fld << 16) | fvol[f * Nfp + a];
-  }
-  __syncthreads();
-  const size_t field = (size_t)K * Np;
-  for (int64_t e = e_begin + blockIdx.x; e < e_end; e += gridDim.x) {
-    const T* qe = q + (size_t)e * Np;
-    T* te = tr + (size_t)e * W;
-    for (int i = threadIdx.x; i < W; i += blockDim.x) {
-      const uint32_t v = s_src[i];
-      te[i] = qe[(v >> 16) * field + (v & 0xffffu)];
-    }
-  }
-}
-
 // Carpenter & Kennedy (1994) five-stage fourth-order 2N-storage coefficients.
 const double kRK4A[5] = {0.0, -567301805773.0 / 1357537059087.0,
                          -2404267990393.0 / 2016746695238.0,
@@ -278,25 +251,10 @@ int launch_extract(bb_solver* s, const void* q, void* tr, cudaStream_t st, int64
                    int64_t e1 = -1) {
   if (e1 < 0) e1 = s->K;
   if (e1 <= e0) return BB_OK;
-  int64_t grid = e1 - e0;
-  if (grid > (int64_t)s->ctx->num_sms * 8) grid = (int64_t)s->ctx->num_sms * 8;
-  const DegTables& t = *s->tab;
-  const size_t smem = (size_t)4 * s->nf * t.Nfp * sizeof(uint32_t);
-#define BB_EXTRACT(T_, NF_)                                                                \
-  extract_traces_kernel<T_, NF_><<<(int)grid, 256, smem, st>>>(t, t.d_words, s->K,         \
-                                                                (const T_*)q, (T_*)tr, e0, e1)
-  if (s->dtype == BB_F64) {
-    if (s->nf == 4) BB_EXTRACT(double, 4);
-    else if (s->nf == 1) BB_EXTRACT(double, 1);
-    else if (s->nf == 3) BB_EXTRACT(double, 3);
-    else BB_EXTRACT(double, 6);
-  } else {
-    if (s->nf == 4) BB_EXTRACT(float, 4);
-    else if (s->nf == 1) BB_EXTRACT(float, 1);
-    else if (s->nf == 3) BB_EXTRACT(float, 3);
-    else BB_EXTRACT(float, 6);
-  }
-#undef BB_EXTRACT
+  if (s->dtype == BB_F64)
+    extract_traces<double>(*s->tab, s->nf, s->K, q, tr, e0, e1, s->ctx->num_sms, st);
+  else
+    extract_traces<float>(*s->tab, s->nf, s->K, q, tr, e0, e1, s->ctx->num_sms, st);
   return bb_check_launch(s->ctx, "extract_traces_kernel");
 }
 
