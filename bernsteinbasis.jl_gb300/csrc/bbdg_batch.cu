@@ -23,7 +23,8 @@
 namespace {
 
 constexpr int kBatchThreads = 256;
-constexpr int kSideStreams = 8;  // streams the fast lanes are spread over
+constexpr int kSideStreams = 8;  // streams the small fast lanes are spread over
+constexpr int kLargeRounds = 2;  // tiles per resident block from which a problem is large
 const double kA[5] = {0.0, -567301805773.0 / 1357537059087.0, -2404267990393.0 / 2016746695238.0,
                       -3550918686646.0 / 2091501179385.0, -1275806237668.0 / 842570457699.0};
 const double kB[5] = {1432997174477.0 / 9575080441755.0, 5161836677717.0 / 13612068292357.0,
@@ -99,6 +100,10 @@ struct bb_batch {
   std::vector<int> epb;          // per problem
   std::vector<int> fast;         // per problem: specialised variant, -1 = generic kernel
   std::vector<const void*> fast_tables;  // its table image
+  // fast lanes that share the GPU on the side streams, and those that fill it by themselves: a
+  // persistent launch gives each block its tiles up front, so a block that another problem's
+  // kernel keeps off its SM ends late by all of its tiles
+  std::vector<int> small, large;
   int nfast = 0, ngeneric = 0;
   std::vector<void*> trace;      // 2 per problem
   void* d_desc = nullptr;
@@ -144,6 +149,8 @@ int build_desc(bb_batch* b) {
   b->fast.assign(np, -1);
   b->fast_tables.assign(np, nullptr);
   b->nfast = b->ngeneric = 0;
+  b->small.clear();
+  b->large.clear();
   for (int p = 0; p < np; ++p) {
     const bb_batch_problem& pr = b->probs[p];
     if (sizeof(T) == 4 && a16(pr.q) && a16(pr.res) && a16(pr.geo) && a16(pr.conn)) {
@@ -157,6 +164,11 @@ int build_desc(bb_batch* b) {
       b->fast_tables[p] = bb_fast_tables(ctx, b->fast[p]);
       if (!b->fast_tables[p]) return bb_fail(ctx, BB_ERR_NOMEM, "table allocation failed");
       ++b->nfast;
+      int e = 0, th = 0;
+      size_t sm = 0;
+      bb_fast_variant_info(b->fast[p], &e, &th, &sm);
+      const int64_t resident = ctx->num_sms * std::min<int64_t>(4, 228 * 1024 / (sm + 1024));
+      (pr.K >= kLargeRounds * e * resident ? b->large : b->small).push_back(p);
     }
   }
   std::vector<BatchDesc<T>> h;
@@ -246,16 +258,15 @@ int launch_fast_lane(bb_batch* b, int p, int s, int par, cudaStream_t st) {
 template <class T>
 int enqueue_batch_step(bb_batch* b, int par, cudaStream_t st) {
   bb_ctx* ctx = b->ctx;
-  const int nside = std::min(b->nfast, kSideStreams);
-  if (nside > 0) {  // fork: the fast lanes start with the step
+  const int nside = (int)std::min<size_t>(b->small.size(), kSideStreams);
+  if (nside > 0) {  // fork: the small fast lanes start with the step
     BB_CUDA(ctx, cudaEventRecord(b->fork_ev, st));
     for (int i = 0; i < nside; ++i) BB_CUDA(ctx, cudaStreamWaitEvent(b->side[i], b->fork_ev, 0));
     int j = 0;
-    for (size_t p = 0; p < b->probs.size(); ++p) {
-      if (b->fast[p] < 0) continue;
+    for (int p : b->small) {
       cudaStream_t ss = b->side[j++ % nside];
       for (int s = 0; s < 5; ++s) {
-        const int rc = launch_fast_lane(b, (int)p, s, par, ss);
+        const int rc = launch_fast_lane(b, p, s, par, ss);
         if (rc) return rc;
       }
     }
@@ -274,6 +285,11 @@ int enqueue_batch_step(bb_batch* b, int par, cudaStream_t st) {
     BB_CUDA(ctx, cudaEventRecord(b->join_ev[i], b->side[i]));
     BB_CUDA(ctx, cudaStreamWaitEvent(st, b->join_ev[i], 0));
   }
+  for (int p : b->large)
+    for (int s = 0; s < 5; ++s) {
+      const int rc = launch_fast_lane(b, p, s, par, st);
+      if (rc) return rc;
+    }
   return BB_OK;
 }
 
