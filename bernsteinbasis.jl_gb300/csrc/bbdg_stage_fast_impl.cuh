@@ -374,6 +374,9 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   auto tile_ne = [=](int t) { return ANY ? min(EPB, (int)K - t * EPB) : EPB; };
   const uint32_t wlim = P.wait_iters ? P.wait_iters : (1u << 24);
   const bool stage = P.mode != 0;
+  // the first stage of a step (rkA = 0) ignores what res holds, and does not read it (a fifth of
+  // that stage's HBM traffic): the update finds zeros in its place
+  const bool use_res = stage && P.rkA != 0.f;
   // element threads: element le, lane u within the element
   const int le = tid / TPE, u = tid - (tid / TPE) * TPE;
   const bool is_elem = tid < NTE;
@@ -446,7 +449,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
 #pragma unroll
     for (int m = 0; m < NF; ++m) {
       prefetch_row(gq + ((size_t)m * K + e0) * NP, EPB * NP);
-      if (stage) prefetch_row(gres + ((size_t)m * K + e0) * NP, EPB * NP);
+      if (use_res) prefetch_row(gres + ((size_t)m * K + e0) * NP, EPB * NP);
     }
     l2_prefetch(ggeo + e0 * BB_GEO_STRIDE, L::GEOBYTES);
     l2_prefetch(gconn + e0 * 4, L::CONNBYTES);
@@ -462,6 +465,8 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
+  if (stage && !use_res)
+    for (int t = tid; t < NF * EPB * NP; t += NT) sRes[t] = 0.f;
   for (int t = tid; t < NZ_W; t += NT)
     sW[((t / (L::NZ * NW)) * L::NPM1P + L::Z0 + (t / NW) % L::NZ) * NW + t % NW] = 0.f;
   __syncthreads();
@@ -476,7 +481,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   if ((bulk ? issuer : !is_elem) && t0 < ntiles) {
     issue_main(t0, 0);
     ++iss0;
-    if (stage) issue_res(t0), ++iss2;
+    if (use_res) issue_res(t0), ++iss2;
     if (t0 + step < ntiles) issue_main(t0 + step, 1), ++iss1;
     if (issuer && t0 + 2 * step < ntiles) prefetch_tile(t0 + 2 * step);
   }
@@ -625,14 +630,14 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     if (!is_elem) {
       if (it > 0) {
         for (int g = 0; g < NG; ++g) nbar_sync(1 + NG + g, GCOUNT);
-        if ((bulk ? issuer : true) && !*vfail && (tnext < ntiles || stage)) {
+        if ((bulk ? issuer : true) && !*vfail && (tnext < ntiles || use_res)) {
           fence_async_smem();  // order the generic-proxy reads before the copies
           if (tnext < ntiles) {
             issue_main(tnext, s ^ 1, P.fault == 1 && it == 1);
             if (s) ++iss0;
             else ++iss1;
           }
-          if (stage) issue_res(tile), ++iss2;
+          if (use_res) issue_res(tile), ++iss2;
           if (issuer && tnext + step < ntiles) prefetch_tile(tnext + step);
         }
       }
@@ -742,7 +747,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
         ph ^= 1u << (s ^ 1);
         if (!*vfail && (!ANY || tnext < mytiles)) flux_tile(tnext, s ^ 1, sX + (s ^ 1) * NCHAIN * NFP);
       }
-      if (stage && !*vfail) {
+      if (use_res && !*vfail) {
         if (!mbar_wait(&bar[2], (ph >> 2) & 1u, wlim)) {
           s_fail = 1;
           atomicOr(P.status, 2);

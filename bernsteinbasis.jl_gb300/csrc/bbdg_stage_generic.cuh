@@ -191,6 +191,7 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
   const int N = P.tab.N, Np = P.tab.Np, NpM1 = P.tab.NpM1, Nfp = P.tab.Nfp;
   const int64_t K = P.K;
   const int epb = P.epb;
+  const bool use_res = P.mode != 0 && P.rkA != T(0);
   const FastDiv by_np(Np), by_npm1(NpM1), by_nfp(Nfp), by_4nfp(4 * Nfp);
     const int64_t e0 = tile * epb;
     const int ne = (int)min64(epb, K - e0);
@@ -392,11 +393,9 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
         const int pf[4] = {(int)(ga.z & 0xffff), (int)(ga.z >> 16), (int)(ga.w & 0xffff),
                            (int)(ga.w >> 16)};
         const size_t at = ((size_t)f0 * K + e0 + le) * Np + n, fs = (size_t)K * Np;
-        T res[FG];
-        if (P.mode != 0) {
+        T res[FG];  // the first stage of a step (rkA = 0) ignores what it holds
 #pragma unroll
-          for (int m = 0; m < FG; ++m) res[m] = P.res[at + m * fs];
-        }
+        for (int m = 0; m < FG; ++m) res[m] = use_res ? P.res[at + m * fs] : T(0);
         T acc[FG];
 #pragma unroll
         for (int m = 0; m < FG; ++m) acc[m] = T(0);
@@ -528,7 +527,7 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
         for (int t = threadIdx.x; t < ne * Np; t += blockDim.x) {
           const int le = by_np.div(t);
           const T rhs = so[t] * sGeo[le * BB_GEO_STRIDE + 9];
-          const T r = P.rkA * gr[t] + P.dt * rhs;
+          const T r = P.rkA * (use_res ? gr[t] : T(0)) + P.dt * rhs;
           const T qn = sq[t] + P.rkB * r;
           gr[t] = r;
           gq[t] = qn;

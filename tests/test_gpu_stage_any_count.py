@@ -80,3 +80,22 @@ def test_high_degrees_equal_the_generic_kernel(cuda, bb, physics, N):
             s.check()
             out.append((rhs, q))
         assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("physics,N,dtype", [("wave", 9, "float32"), ("maxwell", 5, "float32"),
+                                             ("wave", 13, "float32"), ("advection", 4, "float32"),
+                                             ("maxwell", 3, "float64"), ("wave", 20, "float64")])
+def test_a_step_ignores_the_register_it_starts_with(cuda, bb, physics, N, dtype):
+    """The LSRK register is scratch within a step: NaN in it before the step changes nothing."""
+    import torch
+    m = bb.uniform_tet_mesh(3)
+    s = bb.DGSolver(m, N, physics, dtype=getattr(torch, dtype), tau=1.0)
+    gen = torch.Generator(device=cuda).manual_seed(N)
+    q0 = torch.rand((s.nf, m.K, s.Np), generator=gen, device=cuda, dtype=s.dtype)
+    out = []
+    for fill in (0.0, float("nan")):
+        q, r = q0.clone(), torch.full_like(q0, fill)
+        s.run(q, r, 0.1 * s.dt_cfl(), 2)
+        s.check()
+        out.append((q, r))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
