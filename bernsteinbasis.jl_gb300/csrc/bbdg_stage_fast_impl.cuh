@@ -115,17 +115,25 @@ struct FastLayout {
   static constexpr int FVOL_B = VN_B + NPM1 * 8;               // [4][NFP] u16
   static constexpr int FPERM_B = FVOL_B + ((4 * NFP * 2 + 3) / 4 * 4);  // [6][NFP] u16
   static constexpr int FNB_B = FPERM_B + ((6 * NFP * 2 + 3) / 4 * 4);  // [4][6][NFP] u16
-  static constexpr int TF_B = (FNB_B + 24 * NFP * 2 + 15) / 16 * 16;   // [NP] u32 face nodes
-  static constexpr int DEC_B = (TF_B + NP * 4 + 15) / 16 * 16;  // [NP] u16, lift_pair_warp only
+  // The outgoing face traces: with two and more warps per element they are stored face by face from
+  // the updated q in shared memory (three coefficients in four lie on a face, and from the update's
+  // registers that is 16 or 24 scattered predicated stores per coefficient, a tenth of the
+  // instructions; per stage, registers / face by face: Maxwell N = 10, K = 10,368, 154 / 148 us, N = 8,
+  // K = 24,576, 195 / 186; wave N = 15, K = 3,072, 77 / 75); a single warp waits longer for its own
+  // stores than it saves (Maxwell N = 5, K = 24,576, 66.0 / 67.9).
+  static constexpr bool TRACE_SMEM = TPE > 32;
+  static constexpr int TF_B = (FNB_B + 24 * NFP * 2 + 15) / 16 * 16;  // [NP] u32 face nodes
+  static constexpr int DEC_B = (TF_B + (TRACE_SMEM ? 0 : NP * 4) + 15) / 16 * 16;  // [NP] u16
   static constexpr int BAR_B = (DEC_B + (warp_lift<PHYS>(N) ? NP * 2 : 0) + 15) / 16 * 16;  // 4 mbarriers
   static constexpr int TABLES = BAR_B - GA_B;  // the constant tables, one image (fast_image)
   static constexpr int BYTES = BAR_B + 32;
   // element groups for the named-barrier hand-offs between the chain warps and the element
-  // threads: GS elements per group, NG groups, two barriers per group (ids 1..2 NG)
+  // threads: GS elements per group, NG groups, two barriers per group (ids 1..2 NG), and one
+  // among the group's own threads before they store its traces (ids 2 NG + 1..3 NG)
   static constexpr int GS = EPB <= 7 ? 1 : (EPB + 6) / 7;
   static constexpr int NG = EPB / GS;
   static constexpr int GCOUNT = GS * TPE + CHT;  // threads at each hand-off
-  static_assert(EPB % GS == 0 && 2 * NG <= 15, "named barriers 1..15 cover the groups");
+  static_assert(EPB % GS == 0 && 3 * NG <= 15, "named barriers 1..15 cover the groups");
   // resident blocks per SM the register budget is sized for: as many as fit in the SM's shared
   // memory (each block takes 1 KB more than it asks for), up to the four that its 64 named
   // barriers allow. A budget for two blocks left half the SM empty at the low degrees: Maxwell
@@ -133,7 +141,7 @@ struct FastLayout {
   // 168 -> 135.
   static constexpr int FITB = 228 * 1024 / (BYTES + 1024);
   static constexpr int MINB = FITB < 1 ? 1 : FITB < 4 ? FITB : 4;
-  static_assert(NFP < 255, "face node indices are packed in bytes");
+  static_assert(TRACE_SMEM || NFP < 255, "face node indices are packed in bytes");
   static_assert(NPM1P <= 1024 && NPS <= 1024, "w indices and stack slots fit the packed table");
   static_assert(TPE % 32 == 0 && TPE >= 32, "element threads come in whole warps");
 };
@@ -361,7 +369,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
   // partner face nf, orientation o, node a -> volume index of the partner's node
   uint16_t* sFnb = reinterpret_cast<uint16_t*>(smem + L::FNB_B);
   // per coefficient: its node index on faces f0..f3 (one byte each, 0xff = not on the face)
-  uint32_t* sTF = reinterpret_cast<uint32_t*>(smem + L::TF_B);
+  const uint32_t* sTF = reinterpret_cast<const uint32_t*>(smem + L::TF_B);
   const uint16_t* sDec = reinterpret_cast<const uint16_t*>(smem + L::DEC_B);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_B);  // [0],[1] q slots, [2] res,
                                                                  // [3] tables
@@ -884,8 +892,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
 #pragma unroll
           for (int m = 0; m < NF; ++m) grhs_out[((size_t)m * K + e0) * NP + item] = rhs[m];
         } else {
-          // q and res leave straight from registers (coalesced: item runs along the tile),
-          // and so do the outgoing face traces of the coefficients that lie on a face
+          // q and res leave straight from registers (coalesced: item runs along the tile)
           float qn[NF];
 #pragma unroll
           for (int m = 0; m < NF; ++m) {
@@ -894,15 +901,40 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
             gres_out[((size_t)m * K + e0) * NP + item] = rr;
             gq_out[((size_t)m * K + e0) * NP + item] = qn[m];
           }
-          const uint32_t tf = sTF[n];
+          if constexpr (L::TRACE_SMEM) {
 #pragma unroll
-          for (int f = 0; f < 4; ++f) {
-            const uint32_t a = (tf >> (8 * f)) & 0xffu;
-            if (a != 0xffu && leave[f]) {
-              float* dst = P.trace_out + ((size_t)(e0 + le) * 4 + f) * NF * NFP + a;
+            for (int m = 0; m < NF; ++m) sQ[m * EPB * NP + item] = qn[m];
+          } else {
+            const uint32_t tf = sTF[n];
 #pragma unroll
-              for (int m = 0; m < NF; ++m) dst[m * NFP] = qn[m];
+            for (int f = 0; f < 4; ++f) {
+              const uint32_t a = (tf >> (8 * f)) & 0xffu;
+              if (a != 0xffu && leave[f]) {
+                float* dst = P.trace_out + ((size_t)(e0 + le) * 4 + f) * NF * NFP + a;
+#pragma unroll
+                for (int m = 0; m < NF; ++m) dst[m * NFP] = qn[m];
+              }
             }
+          }
+        }
+      }
+    }
+    // TRACE_SMEM: the element's updated q is in its slot (free until the next B->A hand-off), and
+    // each thread stores the nodes of its face in node order
+    if (L::TRACE_SMEM && is_elem && stage && P.trace_out != nullptr) {  // alike for the whole group
+      nbar_sync(1 + 2 * NG + grp, L::GS * TPE);
+      if ((!ANY || tile < mytiles) && !*vfail) {
+        const int64_t nb = (int64_t)((uint32_t)sConn[le * 4 + ff] >> 5);
+        if (nb < e0 || nb >= e0 + EPB) {
+          float* dst = P.trace_out + ((size_t)(e0 + le) * 4 + ff) * NF * NFP;
+          const float* src = sQ + le * NP;
+#pragma unroll
+          for (int r = 0; r < FR; ++r) {
+            const int a = fa0 + r * FT;
+            if (a >= NFP) continue;
+            const float* qa = src + sFvol[ff * NFP + a];
+#pragma unroll
+            for (int m = 0; m < NF; ++m) dst[m * NFP + a] = qa[m * EPB * NP];
           }
         }
       }
@@ -1002,7 +1034,6 @@ std::vector<uint8_t> fast_image() {
   uint16_t* fvol = reinterpret_cast<uint16_t*>(at(L::FVOL_B));
   uint16_t* fperm = reinterpret_cast<uint16_t*>(at(L::FPERM_B));
   uint16_t* fnb = reinterpret_cast<uint16_t*>(at(L::FNB_B));
-  uint32_t* tf = reinterpret_cast<uint32_t*>(at(L::TF_B));
   std::vector<std::array<int, 4>> idx;
   for (int k = 0; k <= N; ++k)
     for (int j = 0; j <= N - k; ++j)
@@ -1018,6 +1049,14 @@ std::vector<uint8_t> fast_image() {
     uint32_t mb[4];
     const int lane = (t % TPE) & 31, phase = L::NZ;  // lanes of one vector-load phase
     const int n0 = t - (lane % phase);
+    if (!L::TRACE_SMEM) {
+      // face nodes: f0 (j=0) at (i,k), f1 (l=0) at (j,k), f2 (i=0) at (j,k), f3 (k=0) at (i,j)
+      const uint32_t a0 = j == 0 ? (uint32_t)ij2(N, i, k) : 0xffu;
+      const uint32_t a1 = l == 0 ? (uint32_t)ij2(N, j, k) : 0xffu;
+      const uint32_t a2 = i == 0 ? (uint32_t)ij2(N, j, k) : 0xffu;
+      const uint32_t a3 = k == 0 ? (uint32_t)ij2(N, i, j) : 0xffu;
+      reinterpret_cast<uint32_t*>(at(L::TF_B))[t] = a0 | (a1 << 8) | (a2 << 16) | (a3 << 24);
+    }
     for (int b = 0; b < 4; ++b) {
       const int x = wnb(t, b);
       if (x >= 0) {
@@ -1044,12 +1083,6 @@ std::vector<uint8_t> fast_image() {
     ga[4 * t + 1] = p0 | (p1 << 10) | (p2 << 20);
     ga[4 * t + 2] = (uint32_t)i | ((uint32_t)j << 8) | ((uint32_t)k << 16) | ((uint32_t)l << 24);
     ga[4 * t + 3] = p3 | (mb[3] << 10);
-    // face nodes: f0 (j=0) at (i,k), f1 (l=0) at (j,k), f2 (i=0) at (j,k), f3 (k=0) at (i,j)
-    const uint32_t a0 = j == 0 ? (uint32_t)ij2(N, i, k) : 0xffu;
-    const uint32_t a1 = l == 0 ? (uint32_t)ij2(N, j, k) : 0xffu;
-    const uint32_t a2 = i == 0 ? (uint32_t)ij2(N, j, k) : 0xffu;
-    const uint32_t a3 = k == 0 ? (uint32_t)ij2(N, i, j) : 0xffu;
-    tf[t] = a0 | (a1 << 8) | (a2 << 16) | (a3 << 24);
   }
   for (int k = 0, t = 0; k < N; ++k)
     for (int j = 0; j < N - k; ++j)
