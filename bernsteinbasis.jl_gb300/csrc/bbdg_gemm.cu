@@ -2,14 +2,14 @@
 //     C[M x N] = alpha * A[M x K] * B[N x K]^T, then a fused epilogue (bbdg_gemm.cuh).
 // A and B are row-major BF16 with K contiguous ("K-major" operands).
 //
-// Persistent, warp-specialised kernel, one CTA per SM (192 threads):
+// Persistent, warp-specialised kernel, one CTA per SM (576 threads):
 //   warp 0      TMA producer: 128 x 64 boxes of A and BN x 64 boxes of B, 128-byte swizzle,
 //               into a STAGES-deep shared-memory ring (mbarrier full / empty pairs);
 //   warp 1      MMA issuer: one thread issues tcgen05.mma (kind::f16, M=128, N=BN, K=16)
 //               into one of two TMEM accumulators and releases ring stages and finished
 //               accumulators with tcgen05.commit;
-//   warps 2-5   epilogue: tcgen05.ld of 32-column chunks (warp w reads TMEM lanes
-//               32(w%4)..+31 = tile rows), staged through a per-warp shared tile so that
+//   warps 2-17  epilogue: tcgen05.ld of 16-column chunks in turn (warp w reads TMEM lanes
+//               32(w%4)..+31 = tile rows; four warps share a quarter), staged through a per-warp shared tile so that
 //               every global store of a warp covers one contiguous row segment (row-major
 //               outputs) or one contiguous column segment (the transposed output).
 // The two accumulators let the epilogue of tile i overlap the main loop of tile i+1.
@@ -104,23 +104,20 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// 32 lanes x 32 bit, 32 consecutive columns per thread (warp w % 4 reads lanes 32(w%4)..+31).
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
+// 32 lanes x 32 bit, 16 consecutive columns per thread (warp w % 4 reads lanes 32(w%4)..+31).
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
-      "%11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, "
-      "%28, %29, %30, %31}, [%32];"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+      "%11, %12, %13, %14, %15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
         "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        "=r"(r[14]), "=r"(r[15])
       : "r"(taddr)
       : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 __device__ __forceinline__ float gelu(float x) {
@@ -160,6 +157,14 @@ __device__ __forceinline__ void st_bf16x4(__nv_bfloat16* p, float4 v) {
   *reinterpret_cast<uint2*>(p) = u;
 }
 
+// Staged 32 x 16 chunk of an epilogue warp: two rows per 128 bytes, the 16-byte groups of a row
+// permuted so that the row-per-lane stores and the row-segment loads touch every bank group
+// once per eight lanes.
+constexpr int kChunk = 16;
+__device__ __forceinline__ int tix(int r, int c) {
+  return r * kChunk + (c ^ (((r >> 1) & 3) << 2));
+}
+
 // One element of the epilogue with compile-time options.
 template <int F>
 __device__ __forceinline__ float epi_value(float x, float b, const GemmEpilogue& ep, size_t off) {
@@ -172,14 +177,14 @@ __device__ __forceinline__ float epi_value(float x, float b, const GemmEpilogue&
   return x;
 }
 
-// Row pass of a staged 32 x 32 chunk (T, pitch 36 floats) with compile-time options: lane l
-// handles columns c0 + 4 (l % 8) .. + 3 of rows 4 i + l / 8, so one warp store writes four
-// contiguous 128-byte (FP32) or 64-byte (BF16) row segments. vec: every output row start is
+// Row pass of a staged 32 x 16 chunk (T, swizzled by tix) with compile-time options: lane l
+// handles columns c0 + 4 (l % 4) .. + 3 of rows 8 i + l / 4, so one warp store writes eight
+// contiguous 64-byte (FP32) or 32-byte (BF16) row segments. vec: every output row start is
 // 16-byte aligned (ldc % 4 == 0 and aligned bases), else the lane falls back to scalars.
 template <int F>
 __device__ __forceinline__ void epi_rows(const GemmEpilogue& ep, float* T, int r0, int c0,
                                          int rows, int lane, bool vec) {
-  const int q = lane >> 3, cg = (lane & 7) * 4;
+  const int q = lane >> 2, cg = (lane & 3) * 4;
   const int c = c0 + cg;
   const int ncol = min(4, ep.N - c);  // columns of this lane inside the matrix (may be <= 0)
   float b[4] = {0.f, 0.f, 0.f, 0.f};
@@ -190,9 +195,9 @@ __device__ __forceinline__ void epi_rows(const GemmEpilogue& ep, float* T, int r
   }
   float g[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int rr = 4 * i + q;
-    float4 x4 = *reinterpret_cast<const float4*>(T + rr * 36 + cg);
+  for (int i = 0; i < 4; ++i) {
+    const int rr = 8 * i + q;
+    float4 x4 = *reinterpret_cast<const float4*>(T + tix(rr, cg));
     if (rr < rows && ncol > 0) {
       const size_t off = (size_t)(r0 + rr) * ep.ldc + c;
       float x[4] = {ep.alpha * x4.x, ep.alpha * x4.y, ep.alpha * x4.z, ep.alpha * x4.w};
@@ -237,13 +242,14 @@ __device__ __forceinline__ void epi_rows(const GemmEpilogue& ep, float* T, int r
         g[2] += x4.z;
         g[3] += x4.w;
       }
-      *reinterpret_cast<float4*>(T + rr * 36 + cg) = x4;
+      *reinterpret_cast<float4*>(T + tix(rr, cg)) = x4;
     }
   }
   if (F & kBgrad) {
-    // lanes l, l+8, l+16, l+24 hold the same columns
+    // lanes of equal l % 4 hold the same columns
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
+      g[j] += __shfl_xor_sync(0xffffffffu, g[j], 4);
       g[j] += __shfl_xor_sync(0xffffffffu, g[j], 8);
       g[j] += __shfl_xor_sync(0xffffffffu, g[j], 16);
     }
@@ -258,12 +264,12 @@ __device__ __forceinline__ void epi_rows(const GemmEpilogue& ep, float* T, int r
 // Row pass with every option read at run time (any alignment, any combination).
 __device__ __forceinline__ void epi_rows_generic(const GemmEpilogue& ep, float* T, int r0,
                                                  int c0, int rows, int lane, bool split) {
-  const int c = c0 + lane;
+  const int cl = lane & (kChunk - 1), c = c0 + cl;
   const bool cin = c < ep.N;
   const float b = (cin && ep.bias) ? ep.bias[c] : 0.0f;
   float gsum = 0.0f;
-  for (int rr = 0; rr < rows; ++rr) {
-    float x = ep.alpha * T[rr * 36 + lane] + b;
+  for (int rr = lane / kChunk; rr < rows; rr += 32 / kChunk) {
+    float x = ep.alpha * T[tix(rr, cl)] + b;
     if (cin) {
       const size_t off = (size_t)(r0 + rr) * ep.ldc + c;
       if (ep.act == 1) {
@@ -279,9 +285,10 @@ __device__ __forceinline__ void epi_rows_generic(const GemmEpilogue& ep, float* 
       if (ep.Cb) ep.Cb[off] = __float2bfloat16_rn(x);
       gsum += x;
     }
-    T[rr * 36 + lane] = x;
+    T[tix(rr, cl)] = x;
   }
-  if (ep.bias_grad && cin) atomicAdd(ep.bias_grad + c, gsum);
+  gsum += __shfl_xor_sync(0xffffffffu, gsum, kChunk);
+  if (ep.bias_grad && cin && lane < kChunk) atomicAdd(ep.bias_grad + c, gsum);
 }
 
 template <int BN_>
@@ -292,10 +299,14 @@ struct GemmCfg {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = (192 * 1024) / STAGE_BYTES;  // 4 or 6
   static constexpr int TMEM_COLS = 2 * BN;               // two FP32 accumulators
-  static constexpr int EPI_WARPS = 4;
+  // EPI_PARTS epilogue warps per 32-row quarter of the accumulator take its 16-column chunks
+  // in turn: the latency of the GELU epilogue, not the MMA, bounds a hidden layer. One warp
+  // per quarter with 32-column chunks: 155 us for the three layers 840-512-512-336 at 24,576
+  // rows; two 103 us; four (16-column chunks keep the staging at 32 KiB) 89 us.
+  static constexpr int EPI_PARTS = 4;
+  static constexpr int EPI_WARPS = 4 * EPI_PARTS;
   static constexpr int THREADS = 64 + 32 * EPI_WARPS;
-  static constexpr int EPI_PITCH = 36;                   // floats; 16-byte rows
-  static constexpr int EPI_BYTES = EPI_WARPS * 32 * EPI_PITCH * 4;
+  static constexpr int EPI_BYTES = EPI_WARPS * 32 * kChunk * 4;
   static constexpr int NBAR = 2 * STAGES + 5;
   static constexpr int SMEM = STAGES * STAGE_BYTES + EPI_BYTES + 8 * NBAR + 16 + 1024;
   // instruction descriptor, kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9 and
@@ -443,7 +454,9 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
     // 16-byte vector stores need 16-byte aligned row starts for every row-major output
     const bool vec = (ep.ldc % 4 == 0) && ((((uintptr_t)ep.Cf | (uintptr_t)ep.Pre) & 15) == 0) &&
                      ((((uintptr_t)ep.Cb) & 7) == 0);
-    float* T = epi + (warp - 2) * 32 * C::EPI_PITCH;
+    const int part = (warp - 2) >> 2;  // chunks part, part + EPI_PARTS, ...
+    constexpr int kStep = C::EPI_PARTS * kChunk;
+    float* T = epi + (warp - 2) * 32 * kChunk;
     int local = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, ++local) {
       int mt, nt, kt0, nkt;
@@ -463,20 +476,20 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
       const int r0 = mt * C::BM + g * 32;
       const int n0 = nt * BN;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        float v[32];
-        tmem_ld32(tmem + ((uint32_t)(g * 32) << 16) + (uint32_t)(a * BN + c0), v);
-        if (c0 + 32 == BN) {
-          // accumulator fully read: hand it back to the MMA warp
+      for (int c0 = part * kChunk; c0 < BN; c0 += kStep) {
+        float v[kChunk];
+        tmem_ld16(tmem + ((uint32_t)(g * 32) << 16) + (uint32_t)(a * BN + c0), v);
+        if (c0 + kStep >= BN) {
+          // this warp's part of the accumulator is read: hand it back to the MMA warp
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(&tempty[a]);
         }
         if (n0 + c0 >= ep.N) continue;
-        // stage the chunk: lane = row, 8 x 16-byte stores (conflict-free with pitch 36)
+        // stage the chunk: lane = row, 4 x 16-byte stores (conflict-free by tix)
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(T + lane * C::EPI_PITCH + j) =
+        for (int j = 0; j < kChunk; j += 4)
+          *reinterpret_cast<float4*>(T + tix(lane, j)) =
               make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
         __syncwarp();
         const int rows = min(32, ep.M - r0);
@@ -486,11 +499,11 @@ __global__ void __launch_bounds__(GemmCfg<BN>::THREADS, 1)
           // column pass: lane owns row r0 + lane; each store covers one column segment
           __syncwarp();
           if (lane < rows) {
-            const int cols = min(32, ep.N - (n0 + c0));
+            const int cols = min(kChunk, ep.N - (n0 + c0));
             __nv_bfloat16* o = ep.CbT + (size_t)(n0 + c0) * ep.ldt + r0 + lane;
 #pragma unroll 8
             for (int j = 0; j < cols; ++j)
-              o[(size_t)j * ep.ldt] = __float2bfloat16_rn(T[lane * C::EPI_PITCH + j]);
+              o[(size_t)j * ep.ldt] = __float2bfloat16_rn(T[tix(lane, j)]);
           }
         }
         __syncwarp();
