@@ -152,6 +152,14 @@ __global__ void transpose_bf16_kernel(const __nv_bfloat16* __restrict__ in, int6
   }
 }
 
+// Elements per block of the closure's gather (features) and update (apply) kernels. The position
+// (field, face, node) of a value is decoded once for all of them, and their loads are in flight
+// together. One element per block with the decoding in 64 bits kept the ALUs busy for 75 us
+// (features) and 29 us (apply) at degree 5, six fields, 24,576 elements; now 34 us and 13 us.
+// Features by 4 instead of 8 elements: 44 against 40 us; apply by 8 instead of 4: 14.6 against 13.
+constexpr int kClosureElems = 8;
+constexpr int kApplyElems = 4;
+
 // Closure features of element e (nf fields, degree N), scaled and rounded to BF16:
 //   [fld][p]        own coefficients, p < Np
 //   [f][fld][a]     the neighbour's coefficients on the shared face f, face node a < Nfp, in
@@ -166,29 +174,48 @@ __global__ void closure_features_kernel(const uint32_t* __restrict__ gtab, int o
   const int nown = nf * Np, nin = nown + 4 * nf * Nfp;
   const uint16_t* fvol = reinterpret_cast<const uint16_t*>(gtab + o_fvol);
   const uint16_t* fperm = reinterpret_cast<const uint16_t*>(gtab + o_fperm);
-  for (int64_t e = blockIdx.x; e < K; e += gridDim.x) {
-    for (int t = threadIdx.x; t < nin; t += blockDim.x) {
-      float val;
-      if (t < nown) {
-        const int fld = t / Np, p = t - fld * Np;
-        val = (float)q[((int64_t)fld * K + e) * Np + p];
-      } else {
-        const int u = t - nown;
-        const int f = u / (nf * Nfp), rest = u - f * nf * Nfp;
-        const int fld = rest / Nfp, a = rest - fld * Nfp;
-        const int32_t c = __ldg(conn + e * 4 + f);
-        const int64_t nbr = (int64_t)((uint32_t)c >> 5);
-        const int nface = (c >> 3) & 3, o = c & 7;
-        if (nbr >= K || o > 5) {
-          atomicOr(status, 1);
-          val = 0.0f;
-        } else {
-          const int vP = fvol[nface * Nfp + fperm[o * Nfp + a]];
-          val = (float)q[((int64_t)fld * K + nbr) * Np + vP];
-        }
+  const int64_t e0 = (int64_t)blockIdx.x * kClosureElems;
+  const int ne = (int)(K - e0 < kClosureElems ? K - e0 : kClosureElems);
+  // per element and face: the neighbour (-1: corrupt connectivity), where its face nodes and the
+  // node permutation of the orientation start
+  __shared__ int s_nbr[kClosureElems][4], s_vol[kClosureElems][4], s_perm[kClosureElems][4];
+  if (threadIdx.x < 4 * kClosureElems) {
+    const int u = threadIdx.x >> 2, f = threadIdx.x & 3;
+    const int32_t c = u < ne ? __ldg(conn + (e0 + u) * 4 + f) : 0;
+    const int64_t nbr = (int64_t)((uint32_t)c >> 5);
+    const int o = c & 7;
+    const bool bad = nbr >= K || o > 5;
+    if (bad) atomicOr(status, 1);
+    s_nbr[u][f] = bad ? -1 : (int)nbr;
+    s_vol[u][f] = ((c >> 3) & 3) * Nfp;
+    s_perm[u][f] = bad ? 0 : o * Nfp;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < nin; t += blockDim.x) {
+    float val[kClosureElems];
+    if (t < nown) {
+      const int fld = t / Np, p = t - fld * Np;
+      const T* src = q + ((int64_t)fld * K + e0) * Np + p;
+#pragma unroll
+      for (int u = 0; u < kClosureElems; ++u) val[u] = u < ne ? (float)src[u * Np] : 0.0f;
+    } else {
+      const int u0 = t - nown;
+      const int f = u0 / (nf * Nfp), rest = u0 - f * nf * Nfp;
+      const int fld = rest / Nfp, a = rest - fld * Nfp;
+      const T* src = q + (int64_t)fld * K * Np;
+      int vP[kClosureElems];
+#pragma unroll
+      for (int u = 0; u < kClosureElems; ++u)
+        vP[u] = __ldg(fvol + s_vol[u][f] + __ldg(fperm + s_perm[u][f] + a));
+#pragma unroll
+      for (int u = 0; u < kClosureElems; ++u) {
+        const int nbr = s_nbr[u][f];
+        val[u] = nbr < 0 ? 0.0f : (float)src[(int64_t)nbr * Np + vP[u]];
       }
-      X[e * nin + t] = __float2bfloat16_rn(val * scale);
     }
+#pragma unroll
+    for (int u = 0; u < kClosureElems; ++u)
+      if (u < ne) X[(e0 + u) * nin + t] = __float2bfloat16_rn(val[u] * scale);
   }
 }
 
@@ -196,15 +223,22 @@ __global__ void closure_features_kernel(const uint32_t* __restrict__ gtab, int o
 template <class T>
 __global__ void closure_apply_kernel(int Np, int64_t K, int nf, float alpha,
                                      const float* __restrict__ Y, T* __restrict__ q) {
-  const int64_t n = K * nf * Np;
   const int nw = nf * Np;
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t e = t / nw;
-    const int j = (int)(t - e * nw);
-    const int fld = j / Np, p = j - fld * Np;
-    const int64_t off = ((int64_t)fld * K + e) * Np + p;
-    q[off] = (T)((float)q[off] + alpha * Y[t]);
+  const int64_t e0 = (int64_t)blockIdx.x * kApplyElems;
+  const int ne = (int)(K - e0 < kApplyElems ? K - e0 : kApplyElems);
+  for (int t = threadIdx.x; t < nw; t += blockDim.x) {
+    const int fld = t / Np, p = t - fld * Np;
+    T* dst = q + ((int64_t)fld * K + e0) * Np + p;
+    const float* src = Y + e0 * nw + t;
+    float y[kApplyElems], v[kApplyElems];
+#pragma unroll
+    for (int u = 0; u < kApplyElems; ++u) {
+      y[u] = u < ne ? src[(int64_t)u * nw] : 0.0f;
+      v[u] = u < ne ? (float)dst[(int64_t)u * Np] : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < kApplyElems; ++u)
+      if (u < ne) dst[(int64_t)u * Np] = (T)(v[u] + alpha * y[u]);
   }
 }
 
@@ -501,13 +535,13 @@ extern "C" int bb_closure_features(bb_ctx* ctx, int N, int64_t K, int nf, const 
   int* status = bb_ctx_status_word(ctx);
   if (!status) return bb_fail(ctx, BB_ERR_NOMEM, "status word allocation failed");
   cudaStream_t st = (cudaStream_t)stream;
-  const int grid = (int)std::min<int64_t>(K, (int64_t)ctx->num_sms * 32);
+  const int64_t grid = (K + kClosureElems - 1) / kClosureElems;
   if (dtype == BB_F64)
-    closure_features_kernel<double><<<grid, 256, 0, st>>>(t->d_words, t->o_fvol, t->o_fperm, N, K,
+    closure_features_kernel<double><<<(unsigned)grid, 256, 0, st>>>(t->d_words, t->o_fvol, t->o_fperm, N, K,
                                                           nf, conn, (const double*)q, scale,
                                                           (__nv_bfloat16*)X, status);
   else
-    closure_features_kernel<float><<<grid, 256, 0, st>>>(t->d_words, t->o_fvol, t->o_fperm, N, K,
+    closure_features_kernel<float><<<(unsigned)grid, 256, 0, st>>>(t->d_words, t->o_fvol, t->o_fperm, N, K,
                                                          nf, conn, (const float*)q, scale,
                                                          (__nv_bfloat16*)X, status);
   rc = bb_check_launch(ctx, "closure_features_kernel");
@@ -525,11 +559,11 @@ extern "C" int bb_closure_apply(bb_ctx* ctx, int N, int64_t K, int nf, int dtype
   if (rc) return rc;
   if (K == 0) return BB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const int64_t n = K * nf * np3(N);
-  const int grid = grid_for(ctx, n, 256);
+  const int64_t grid = (K + kApplyElems - 1) / kApplyElems;
+  if (grid > INT32_MAX) return bb_fail(ctx, BB_ERR_ARG, "bad argument to bb_closure_apply");
   if (dtype == BB_F64)
-    closure_apply_kernel<double><<<grid, 256, 0, st>>>(np3(N), K, nf, alpha, Y, (double*)q);
+    closure_apply_kernel<double><<<(unsigned)grid, 256, 0, st>>>(np3(N), K, nf, alpha, Y, (double*)q);
   else
-    closure_apply_kernel<float><<<grid, 256, 0, st>>>(np3(N), K, nf, alpha, Y, (float*)q);
+    closure_apply_kernel<float><<<(unsigned)grid, 256, 0, st>>>(np3(N), K, nf, alpha, Y, (float*)q);
   return bb_check_launch(ctx, "closure_apply_kernel");
 }
