@@ -535,16 +535,16 @@ int ensure_host_streams(bb_solver* s) {
 }
 
 // bb_lsrk_run_host's schedule (HostPlan without its events) for K elements in tiles of epb,
-// from a host copy of the packed connectivity: up to kHostMaxChunks chunks of at least 8
+// from a host copy of the packed connectivity: up to `most` chunks of at least 8
 // tiles, the chunk neighbour graph (chunk c touches chunk d when an element of c has a face
 // neighbour in d; entries that name no element, which the kernels report, add no edge), the
 // upload order (breadth-first from chunk 0, lower chunks first) and the launch order and
 // waits of each stage.
 constexpr int kHostMaxChunks = BB_HOST_MAX_CHUNKS;
 static_assert(kHostMaxChunks <= 64, "chunk neighbour sets are 64-bit masks");
-void plan_schedule(int64_t K, int epb, const int32_t* conn, HostPlan* P) {
+void plan_schedule(int64_t K, int epb, const int32_t* conn, int most, HostPlan* P) {
   const int64_t ntiles = (K + epb - 1) / epb;
-  const int C = (int)std::min<int64_t>(kHostMaxChunks, std::max<int64_t>(1, ntiles / 8));
+  const int C = (int)std::min<int64_t>(most, std::max<int64_t>(1, ntiles / 8));
   P->epb = epb;
   P->C = C;
   P->tb.assign(C + 1, 0);
@@ -613,6 +613,19 @@ void plan_schedule(int64_t K, int epb, const int32_t* conn, HostPlan* P) {
   }
 }
 
+// The most chunks for a state of this size. A chunk costs about 10 us of launches and copies on
+// the critical path; the pipeline's fill and drain cost copies of a few chunks, bytes / C: the
+// best C grows with the root of the size. One step, us, with 1 / 8 / 12 / 16 / 24 chunks: wave
+// degree 3, 1 MB: 52 / 129 / 208 / 234 / 345; degree 9, 10.8 MB: 218 / 271 / 353 / 385 / 560;
+// degree 5, 22 MB: 437 / 396 / 404 / 430 / 541; degree 9, 86.5 MB: 1494 / 1253 / 1147 / 1111 /
+// 1268; 692 MB (12 / 16 / 24): 7996 / 7283 / 6547. Below eight chunks the overlap pays for no
+// more than the chunks cost.
+int host_chunks(const bb_solver* s) {
+  const double bytes = (double)s->nf * s->K * s->tab->Np * dtype_size(s->dtype);
+  const int c = (int)std::min<double>(kHostMaxChunks, std::sqrt(bytes / (320 << 10)));
+  return c < 8 ? 1 : c;
+}
+
 // Builds (or keeps) bb_lsrk_run_host's schedule for the solver's tile size, with its events;
 // the connectivity is read once from the device.
 int build_host_plan(bb_solver* s) {
@@ -638,7 +651,7 @@ int build_host_plan(bb_solver* s) {
     return bb_fail(s->ctx, BB_ERR_CUDA, "connectivity download failed");
   }
   try {
-    plan_schedule(s->K, s->epb, conn.data(), P);
+    plan_schedule(s->K, s->epb, conn.data(), host_chunks(s), P);
   } catch (const std::bad_alloc&) {
     delete P;
     return bb_fail(s->ctx, BB_ERR_NOMEM, "host schedule allocation failed");
@@ -656,13 +669,22 @@ int build_host_plan(bb_solver* s) {
   return BB_OK;
 }
 
-// Copies field slices of elements [e0, e1) between the device state and a host buffer.
+// Copies elements [e0, e1) of all fields between the device state and a host buffer: one
+// strided copy (a row per field). The copies of many small chunks are bound by the cost of each
+// copy: 86.5 MB up in 64 chunks takes 0.97 ms as four copies a chunk and 0.54 ms as one. A
+// field longer than the largest pitch is copied by itself.
 int copy_range(bb_solver* s, char* dst, const char* src, int64_t e0, int64_t e1,
                cudaMemcpyKind kind, cudaStream_t st) {
   const size_t row = (size_t)s->tab->Np * dtype_size(s->dtype);
+  const size_t pitch = (size_t)s->K * row, width = (size_t)(e1 - e0) * row;
+  if (pitch <= (size_t)INT32_MAX) {
+    BB_CUDA(s->ctx, cudaMemcpy2DAsync(dst + (size_t)e0 * row, pitch, src + (size_t)e0 * row, pitch,
+                                      width, s->nf, kind, st));
+    return BB_OK;
+  }
   for (int f = 0; f < s->nf; ++f) {
     const size_t off = ((size_t)f * s->K + e0) * row;
-    BB_CUDA(s->ctx, cudaMemcpyAsync(dst + off, src + off, (size_t)(e1 - e0) * row, kind, st));
+    BB_CUDA(s->ctx, cudaMemcpyAsync(dst + off, src + off, width, kind, st));
   }
   return BB_OK;
 }
@@ -897,7 +919,7 @@ extern "C" int bb_lsrk_run_host(bb_solver* s, double dt, int nsteps, const void*
 }
 
 // The schedule bb_lsrk_run_host uses for K elements in tiles of epb with this (host) packed
-// connectivity; host-only. Arrays hold at least BB_HOST_MAX_CHUNKS (+1 for chunk_tiles)
+// connectivity and a state that is large enough for the most chunks; host-only. Arrays hold at least BB_HOST_MAX_CHUNKS (+1 for chunk_tiles)
 // entries per row: chunk_tiles[c] = first tile of chunk c (chunk_tiles[C] = tile count),
 // up = upload order, order[s*max + i] = i-th chunk stage s launches, ready0[i] = last upload
 // position order[0][i] needs, wait[s*max + i] = launch of stage s-1 that order[s][i] waits for.
@@ -909,7 +931,7 @@ extern "C" int bb_host_schedule(int64_t K, int epb, const int32_t* conn_host, in
     return BB_ERR_ARG;
   HostPlan P;
   try {
-    plan_schedule(K, epb, conn_host, &P);
+    plan_schedule(K, epb, conn_host, kHostMaxChunks, &P);
   } catch (const std::bad_alloc&) {
     return BB_ERR_NOMEM;
   }
