@@ -1,9 +1,10 @@
 // Batched persistent stage kernel: many independent wave / Maxwell problems of uneven
 // degree N and element count K advance together.
 //
-// FP32 problems with a degree-specialised stage kernel for their (N, physics) and element
-// count ("fast lanes") run that kernel, each problem its own persistent launch per stage on
-// one of several side streams, so that small problems share the GPU. The other problems run
+// FP32 problems with a degree-specialised stage kernel for their (N, physics) ("fast lanes")
+// run that kernel, each problem its own persistent launch per stage: the small ones on one of
+// several side streams, so that they share the GPU, those that fill it by themselves one after
+// the other on the caller's stream. The other problems run
 // the batched generic kernel: work items are (problem, element tile) pairs, numbered problem
 // by problem; the blocks of a persistent grid draw items from a device counter (one 64-bit
 // atomicAdd per item, no spinning) and run the generic stage tile (bbdg_stage_generic.cuh)

@@ -4,7 +4,8 @@
 //
 // Same algorithm and data layout as the generic stage kernel (bbdg_solver.cu) with the
 // degree N a compile-time constant, which turns every multi-index computation into an
-// immediate and lets one thread run a whole face lift chain in registers:
+// immediate and lets one thread run a whole face lift chain in registers (high degrees: a pair
+// of warps works level by level on a face, lift_pair_warp):
 //
 //   lift, per face f and chain c (src/BernsteinLift.jl:139-164):
 //     E0 = L0 x,  L0 = (N+1)^2/2 R_{N+1} E_{N->N+1}, applied as its 7-point stencil
@@ -26,7 +27,8 @@
 // loop in two phases: (A) the chain warp lifts tile i while the element threads form the
 // volume term of tile i and the interface flux of tile i+1 (double-buffered chain inputs);
 // (B) the element threads gather the lift stacks, add the volume term and apply the LSRK
-// update, storing q, res and the outgoing face traces straight to HBM. q, geometry and
+// update, storing q and res straight to HBM, and the outgoing face traces too or, with
+// more than one warp per element, face by face from shared memory. q, geometry and
 // connectivity of tile i+2 and res of tile i+1 arrive by bulk copies (cp.async.bulk,
 // mbarrier completion, bounded waits) while tiles i and i+1 are being worked on.
 #include <algorithm>

@@ -10,9 +10,10 @@
 //   3. volume term (3d_wave.jl:59-79): the geometric combination of Dr, Ds, Dt is applied
 //      as sum_b alpha_b w(alpha - e_b), w(beta) = sum_a g_a x(beta + e_a), g the barycentric
 //      weights of the physical derivative (Dr = (D0 - D3)/2 etc.)
-//   4. lift of the four face fluxes (src/BernsteinLift.jl:139-220), accumulated in place
-//   5. divide by J, LSRK update res = A res + dt rhs, q += B res; write q, res and the
-//      tile's outgoing traces
+//   4. lift of the four face fluxes (src/BernsteinLift.jl:139-220): whole stacks where
+//      they fit in shared memory, else accumulated level by level
+//   5. gather of the stacks, divide by J, LSRK update res = A res + dt rhs, q += B res; write
+//      q, res and the tile's outgoing traces
 // q and res are updated in place: no block reads another tile's q, so there is no race.
 #pragma once
 
