@@ -300,7 +300,14 @@ int batch_extract(bb_batch* b, cudaStream_t st) {
     const bb_batch_problem& pr = b->probs[p];
     const DegTables& t = *b->tabs[p];
     const int nf = physics_nf(pr.physics);
-    extract_traces<T>(t, nf, pr.K, pr.q, b->trace[2 * p], 0, pr.K, b->ctx->num_sms, st);
+    int epb = b->epb[p];  // of the kernel that will read them
+    if (b->fast[p] >= 0) {
+      int threads = 0;
+      size_t smem = 0;
+      bb_fast_variant_info(b->fast[p], &epb, &threads, &smem);
+    }
+    extract_traces<T>(t, nf, pr.K, pr.conn, epb, pr.q, b->trace[2 * p], 0, pr.K, b->ctx->num_sms,
+                      st);
     int rc = bb_check_launch(b->ctx, "extract_traces_kernel");
     if (rc) return rc;
   }

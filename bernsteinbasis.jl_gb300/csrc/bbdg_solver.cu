@@ -252,9 +252,11 @@ int launch_extract(bb_solver* s, const void* q, void* tr, cudaStream_t st, int64
   if (e1 < 0) e1 = s->K;
   if (e1 <= e0) return BB_OK;
   if (s->dtype == BB_F64)
-    extract_traces<double>(*s->tab, s->nf, s->K, q, tr, e0, e1, s->ctx->num_sms, st);
+    extract_traces<double>(*s->tab, s->nf, s->K, s->conn, s->epb, q, tr, e0, e1,
+                           s->ctx->num_sms, st);
   else
-    extract_traces<float>(*s->tab, s->nf, s->K, q, tr, e0, e1, s->ctx->num_sms, st);
+    extract_traces<float>(*s->tab, s->nf, s->K, s->conn, s->epb, q, tr, e0, e1,
+                          s->ctx->num_sms, st);
   return bb_check_launch(s->ctx, "extract_traces_kernel");
 }
 

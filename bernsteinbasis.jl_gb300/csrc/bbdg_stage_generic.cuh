@@ -543,25 +543,27 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
 }
 
 // ---- traces of a whole state ------------------------------------------------------------
-// Writes every face trace (all faces) of elements [e_begin, e_end) of q into the trace buffer.
+// Writes the traces of the faces that leave their tile (of epb elements, from element 0 on) of
+// elements [e_begin, e_end) of q into the trace buffer: the stage kernels read no others.
 // An element's 4 NF Nfp trace entries are contiguous in the buffer; each block first decodes
 // entry i into (field, volume node) once (shared table). Then each thread gathers four entries at
 // a time from the element's field rows and stores them at once, over kExtractElems elements per
 // turn, so that several gathers are in flight (wave N = 9, K = 196,608: one entry at a time, element
-// after element, 300 us; HBM floor 204).
+// after element, 300 us; four at a time 250; without the faces inside a tile, a third of them at
+// four elements a tile, 205. All faces' traffic at the HBM rate: 204).
 constexpr int kExtractElems = 8;
 
 template <class T, int NF>
 __global__ void __launch_bounds__(256)
     extract_traces_kernel(DegTables tab, const uint32_t* __restrict__ gtab, int64_t K,
-                          const T* __restrict__ q, T* __restrict__ tr, int64_t e_begin,
-                          int64_t e_end) {
-  extern __shared__ uint32_t s_src[];  // entry i: field << 16 | volume node
+                          const int32_t* __restrict__ conn, int epb, const T* __restrict__ q,
+                          T* __restrict__ tr, int64_t e_begin, int64_t e_end) {
+  extern __shared__ uint32_t s_src[];  // entry i: face << 20 | field << 16 | volume node
   const int Np = tab.Np, Nfp = tab.Nfp, W = 4 * NF * Nfp;
   const uint16_t* fvol = reinterpret_cast<const uint16_t*>(gtab + tab.o_fvol);
   for (int i = threadIdx.x; i < W; i += blockDim.x) {
     const int f = i / (NF * Nfp), rem = i - f * NF * Nfp, fld = rem / Nfp, a = rem - fld * Nfp;
-    s_src[i] = ((uint32_t)fld << 16) | fvol[f * Nfp + a];
+    s_src[i] = ((uint32_t)f << 20) | ((uint32_t)fld << 16) | fvol[f * Nfp + a];
   }
   __syncthreads();
   const size_t field = (size_t)K * Np;
@@ -573,8 +575,15 @@ __global__ void __launch_bounds__(256)
     for (int it = threadIdx.x; it < ne * Q; it += blockDim.x) {
       const int le = by_q.div(it), g = it - le * Q;
       const uint4 v = reinterpret_cast<const uint4*>(s_src)[g];
-      const T* qe = q + (size_t)(e0 + le) * Np;
-      auto at = [&](uint32_t x) { return __ldg(qe + (x >> 16) * field + (x & 0xffffu)); };
+      const int64_t e = e0 + le;
+      auto leaves = [&](uint32_t f) {
+        const int64_t nbr = (int64_t)((uint32_t)__ldg(conn + e * 4 + f) >> 5);
+        const int64_t first = e - (uint32_t)e % (uint32_t)epb;  // e < 2^27
+        return nbr < first || nbr >= first + epb;
+      };
+      if (!leaves(v.x >> 20) && (v.w >> 20 == v.x >> 20 || !leaves(v.w >> 20))) continue;
+      const T* qe = q + (size_t)e * Np;
+      auto at = [&](uint32_t x) { return __ldg(qe + ((x >> 16) & 15u) * field + (x & 0xffffu)); };
       T* te = tr + (size_t)(e0 + le) * W + 4 * g;
       if constexpr (sizeof(T) == 4) {
         *reinterpret_cast<float4*>(te) = make_float4(at(v.x), at(v.y), at(v.z), at(v.w));
@@ -588,13 +597,14 @@ __global__ void __launch_bounds__(256)
 
 // Launches it for elements [e0, e1) of an nf-field state; tr 16-byte aligned.
 template <class T>
-void extract_traces(const DegTables& t, int nf, int64_t K, const void* q, void* tr, int64_t e0,
-                    int64_t e1, int num_sms, cudaStream_t st) {
+void extract_traces(const DegTables& t, int nf, int64_t K, const int32_t* conn, int epb,
+                    const void* q, void* tr, int64_t e0, int64_t e1, int num_sms,
+                    cudaStream_t st) {
   const int64_t turns = (e1 - e0 + kExtractElems - 1) / kExtractElems;
   const int grid = (int)min64(turns, (int64_t)num_sms * 8);
   const size_t smem = (size_t)4 * nf * t.Nfp * sizeof(uint32_t);
   auto go = [&](auto kern) {
-    kern<<<grid, 256, smem, st>>>(t, t.d_words, K, (const T*)q, (T*)tr, e0, e1);
+    kern<<<grid, 256, smem, st>>>(t, t.d_words, K, conn, epb, (const T*)q, (T*)tr, e0, e1);
   };
   if (nf == 4) go(extract_traces_kernel<T, 4>);
   else if (nf == 1) go(extract_traces_kernel<T, 1>);
