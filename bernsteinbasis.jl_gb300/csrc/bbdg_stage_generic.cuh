@@ -550,7 +550,7 @@ __device__ void generic_stage_tile(const StageParams<T>& P, const TileLayout& L,
 // a time from the element's field rows and stores them at once, over kExtractElems elements per
 // turn, so that several gathers are in flight (wave N = 9, K = 196,608: one entry at a time, element
 // after element, 300 us; four at a time 250; without the faces inside a tile, a third of them at
-// four elements a tile, 205. All faces' traffic at the HBM rate: 204).
+// four elements a tile, about 205. All faces' traffic at the HBM rate: 204).
 constexpr int kExtractElems = 8;
 
 template <class T, int NF>

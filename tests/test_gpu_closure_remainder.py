@@ -12,8 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _face_tables(bb, N):
-    """Volume index of face f's node m, and the node pairing of each orientation, read from the
-    connectivity of a mesh by matching the physical face points."""
+    """Volume index of face f's node m (face-local (a, b), b outer)."""
     from oracle import dense
     idx = {t[:3]: n for n, t in enumerate(dense.lut3(N))}
     faces = np.zeros((4, bb.np2(N)), np.int64)
