@@ -36,12 +36,13 @@ import numpy as np  # noqa: E402
 N_DEG = 9
 N_HEX = 32
 NF = 4
-# algorithmic bytes per element per RK stage (FP32): read q, read res, write res, write q
-# (4 nf Np s) + neighbour traces (4 nf Nfp s) + geometry (22 scalars) + connectivity (4 int32)
+# algorithmic bytes per element per RK stage (FP32), the mean over a step's five: read q, write
+# res, write q (3 nf Np s), read res (nf Np s, in four of them: the first stage's coefficient is
+# zero) + neighbour traces (4 nf Nfp s) + geometry (22 scalars) + connectivity (4 int32)
 def stage_bytes_per_element(N=N_DEG, s=4):
     Np = (N + 1) * (N + 2) * (N + 3) // 6
     Nfp = (N + 1) * (N + 2) // 2
-    return 4 * NF * Np * s + 4 * NF * Nfp * s + 22 * s + 16
+    return (3 + 4 / 5) * NF * Np * s + 4 * NF * Nfp * s + 22 * s + 16
 
 
 def peaks():
