@@ -20,6 +20,7 @@
 #include "bbdg_internal.cuh"
 #include "bbdg_stage_fast.cuh"
 #include "bbdg_stage_generic.cuh"
+#include "bbdg_upload.cuh"
 
 namespace {
 
@@ -213,7 +214,7 @@ int build_desc(bb_batch* b) {
   if (!b->d_desc) {
     BB_CUDA(ctx, cudaMalloc(&b->d_desc, sizeof(BatchDesc<T>) * np));
   }
-  BB_CUDA(ctx, cudaMemcpy(b->d_desc, h.data(), sizeof(BatchDesc<T>) * h.size(), cudaMemcpyHostToDevice));
+  BB_CUDA(ctx, upload_bytes(ctx->device, b->d_desc, h.data(), sizeof(BatchDesc<T>) * h.size()));
   BB_CUDA(ctx, cudaFuncSetAttribute(batch_stage_kernel<T>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;

@@ -8,6 +8,7 @@
 #include <cstring>
 
 #include "bbdg_internal.cuh"
+#include "bbdg_upload.cuh"
 
 // -------------------------------------------------------------------------------------
 // context
@@ -197,10 +198,8 @@ const DegTables* bb_tables(bb_ctx* ctx, int N) {
     }
   // (the lift weights l_j(N), constants.jl:10-12, are carried by the chain recursion:
   // no table of them is needed)
-  bool ok = cudaMalloc(&t->d_words, sizeof(uint32_t) * off) == cudaSuccess &&
-            cudaMemcpy(t->d_words, w.data(), sizeof(uint32_t) * off, cudaMemcpyHostToDevice) ==
-                cudaSuccess;
-  if (!ok) {
+  t->d_words = (uint32_t*)upload_table(ctx->device, w.data(), sizeof(uint32_t) * off);
+  if (!t->d_words) {
     free_tables(t);
     return nullptr;
   }

@@ -2,6 +2,7 @@
 // by variant index. The kernels themselves are instantiated in bbdg_stage_fast_v*.cu.
 #include "bbdg_stage_fast_impl.cuh"
 #include "bbdg_stage_fast_variants.h"
+#include "bbdg_upload.cuh"
 
 using bbfast::FastLayout;
 #define BB_EXTERN(n_, p_, e_, t_) \
@@ -58,22 +59,22 @@ extern "C" int bb_fast_variant(int idx, int* N, int* physics, int* epb, int* thr
 const void* bb_fast_tables(bb_ctx* ctx, int idx) {
   std::lock_guard<std::mutex> lock(ctx->mu);
   if (idx < 0) return nullptr;
-  if ((size_t)idx >= ctx->fast_tabs.size()) ctx->fast_tabs.resize(idx + 1, nullptr);
-  void*& d = ctx->fast_tabs[idx];
-  if (d) return d;
-  std::vector<uint8_t> img;
-  int i = 0;
+  try {
+    if ((size_t)idx >= ctx->fast_tabs.size()) ctx->fast_tabs.resize(idx + 1, nullptr);
+    void*& d = ctx->fast_tabs[idx];
+    if (d) return d;
+    std::vector<uint8_t> img;
+    int i = 0;
 #define BB_IMAGE(n_, p_, e_, t_)                                     \
   if (idx == i) img = bbfast::FastKernel<n_, p_, e_, t_>::image();   \
   ++i;
-  BB_FAST_VARIANTS(BB_IMAGE)
+    BB_FAST_VARIANTS(BB_IMAGE)
 #undef BB_IMAGE
-  if (img.empty() || cudaMalloc(&d, img.size()) != cudaSuccess) return d = nullptr;
-  if (cudaMemcpy(d, img.data(), img.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaFree(d);
-    d = nullptr;
+    if (!img.empty()) d = upload_table(ctx->device, img.data(), img.size());
+    return d;
+  } catch (const std::bad_alloc&) {  // host memory: no exception leaves the C ABI's calls
+    return nullptr;
   }
-  return d;
 }
 
 int bb_fast_launch(int idx, const FastLaunch& fl, const FastStageParams& P, cudaStream_t st) {

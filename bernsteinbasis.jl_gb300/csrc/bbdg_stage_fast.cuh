@@ -39,8 +39,8 @@ struct FastLaunch {
 // Index of the compiled variant for (N, physics, elements per block, threads), 0 = any; -1 if
 // none. Any element count will do: the last tile may be partial.
 int bb_fast_find(int N, int physics, int epb, int threads);
-// The variant's constant tables on the context's device, made on first use and freed with the
-// context; nullptr when out of memory. Not to be called while a stream is being captured.
+// The variant's constant tables on the context's device (whichever device is current), complete
+// for any stream, made on first use and freed with the context; nullptr when out of memory.
 struct bb_ctx;
 const void* bb_fast_tables(bb_ctx* ctx, int idx);
 int bb_fast_variant_info(int idx, int* epb, int* threads, size_t* smem);
