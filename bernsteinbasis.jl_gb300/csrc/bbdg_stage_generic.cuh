@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(256)
     extract_traces_kernel(DegTables tab, const uint32_t* __restrict__ gtab, int64_t K,
                           const int32_t* __restrict__ conn, int epb, const T* __restrict__ q,
                           T* __restrict__ tr, int64_t e_begin, int64_t e_end) {
-  extern __shared__ uint32_t s_src[];  // entry i: face << 20 | field << 16 | volume node
+  extern __shared__ __align__(16) uint32_t s_src[];  // entry i: face << 20 | field << 16 | volume node
   const int Np = tab.Np, Nfp = tab.Nfp, W = 4 * NF * Nfp;
   const uint16_t* fvol = reinterpret_cast<const uint16_t*>(gtab + tab.o_fvol);
   for (int i = threadIdx.x; i < W; i += blockDim.x) {
