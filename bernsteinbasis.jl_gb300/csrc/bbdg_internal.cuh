@@ -70,7 +70,6 @@ struct DegTables {
                      // starts at np3(n-1)
   int o_fvol = 0;    // 4*Nfp uint16: face node -> volume index
   int o_fperm = 0;   // 6*Nfp uint16: face node -> neighbour face node, per orientation
-  int o_fstack = 0;  // 4*Np uint16: face f's lift stack entry (layer, node) -> volume index
   int nwords = 0;
   // past the nwords that blocks copy to shared memory:
   int o_gather = 0;  // Np x 4: per coefficient the degree N-1 indices of alpha - e_b (b = 0..3)
@@ -82,7 +81,7 @@ struct DegTables {
 // (shared-memory sizes of a tile are computed from it before the tables exist).
 inline int deg_table_words(int N) {
   return np3(N) + np3(N - 1) + (np3(N + 1) + 1) / 2 + (4 * np2(N) + 1) / 2 +
-         (6 * np2(N) + 1) / 2 + (4 * np3(N) + 1) / 2;
+         (6 * np2(N) + 1) / 2;
 }
 
 // Orientation codes: face vertex m of this side is face vertex PERMS[o][m] of the partner,
@@ -174,7 +173,6 @@ struct SmemTables {
   const uint16_t* node2;
   const uint16_t* fvol;
   const uint16_t* fperm;
-  const uint16_t* fstack;
 };
 
 // Shared-memory view of tables already copied to `s`.
@@ -185,7 +183,6 @@ __device__ __forceinline__ SmemTables tables_view(const DegTables& t, const uint
   r.node2 = reinterpret_cast<const uint16_t*>(s + t.o_node2);
   r.fvol = reinterpret_cast<const uint16_t*>(s + t.o_fvol);
   r.fperm = reinterpret_cast<const uint16_t*>(s + t.o_fperm);
-  r.fstack = reinterpret_cast<const uint16_t*>(s + t.o_fstack);
   return r;
 }
 
@@ -199,7 +196,6 @@ __device__ __forceinline__ SmemTables load_tables(const DegTables& t, const uint
   r.node2 = reinterpret_cast<const uint16_t*>(s + t.o_node2);
   r.fvol = reinterpret_cast<const uint16_t*>(s + t.o_fvol);
   r.fperm = reinterpret_cast<const uint16_t*>(s + t.o_fperm);
-  r.fstack = reinterpret_cast<const uint16_t*>(s + t.o_fstack);
   return r;
 }
 
@@ -229,22 +225,6 @@ __device__ __forceinline__ void copy_g2s(T* __restrict__ s, const T* __restrict_
     for (int t = nv * W + threadIdx.x; t < n; t += blockDim.x) s[t] = __ldg(g + t);
   } else {
     for (int t = threadIdx.x; t < n; t += blockDim.x) s[t] = __ldg(g + t);
-  }
-}
-
-// Block-cooperative copy shared -> global.
-template <class T>
-__device__ __forceinline__ void copy_s2g(T* __restrict__ g, const T* __restrict__ s, int n) {
-  using V = typename VecOf<T>::type;
-  constexpr int W = VecOf<T>::width;
-  if ((((uintptr_t)g | (uintptr_t)s) & 15) == 0) {
-    const int nv = n / W;
-    V* gv = reinterpret_cast<V*>(g);
-    const V* sv = reinterpret_cast<const V*>(s);
-    for (int t = threadIdx.x; t < nv; t += blockDim.x) gv[t] = sv[t];
-    for (int t = nv * W + threadIdx.x; t < n; t += blockDim.x) g[t] = s[t];
-  } else {
-    for (int t = threadIdx.x; t < n; t += blockDim.x) g[t] = s[t];
   }
 }
 
@@ -344,10 +324,9 @@ __device__ __forceinline__ void maxwell_curl(T (&w)[6], T gx, T gy, T gz, T Hx, 
 // L0 x at face node (i, j) of degree N, k = N - i - j: the 7-point stencil of
 // (N+1)^2/2 R_{N+1} E_{N->N+1} (src/BernsteinLift.jl:100-125 then :66-90 with the L0
 // scaling), x in the 2D layout of degree N with row offsets rb (row j), rbn (row j+1) and
-// rbp (row j-1). Shared by the level-parallel and the chain-per-thread lifts. In double the
-// halving is folded into the stencil weights (c/2 instead of a final product by 1/2): every
-// partial sum is then exactly half of the unhalved one, so the bits are the same and the
-// FP64 pipe does one product less per point.
+// rbp (row j-1). In double the halving is folded into the stencil weights (c/2 instead of a
+// final product by 1/2): every partial sum is then exactly half of the unhalved one, so the bits
+// are the same and the FP64 pipe does one product less per point.
 template <class T>
 __device__ __forceinline__ T l0_point(int i, int j, int k, const T* x, int rb, int rbn, int rbp) {
   constexpr bool H = sizeof(T) == 8;
