@@ -491,12 +491,12 @@ static int launch_lift(bb_ctx* ctx, const DegTables* t, int64_t K, int nfaces, c
     if (rc >= 0) return rc;  // otherwise no specialised kernel for this degree
   }
   // the most elements (up to 16) within 54 KB, four blocks per SM (FP64, N = 7: 284 / 270 / 312 us
-  // for 60,001 columns with 36 / 54 / 110 KB)
+  // for 60,001 columns with 36 / 54 / 110 KB), that leave two blocks for every SM
   int epb = 16;
   size_t smem = 0;
   for (; epb >= 1; epb /= 2) {
     smem = align16(sizeof(T) * lift_scalars(*t, nfaces, epb)) + 4 * (size_t)t->nwords;
-    if (smem <= 54 * 1024 || epb == 1) break;
+    if ((smem <= 54 * 1024 && (K + epb - 1) / epb >= 2 * ctx->num_sms) || epb == 1) break;
   }
   if (smem > ctx->smem_optin) return bb_fail(ctx, BB_ERR_ARG, "degree too large for lift tile");
   BB_CUDA(ctx, cudaFuncSetAttribute(lift_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
