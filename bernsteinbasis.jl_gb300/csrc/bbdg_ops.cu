@@ -613,10 +613,23 @@ extern "C" int bb_fused_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const vo
   // The gradient and lift calls back to back. One launch that read each input once was slower in
   // both precisions: FP64 is bound by its pipe (60,001 columns, N = 7: 505 us fused, 192 + 270
   // apart), FP32 has specialised kernels, and above N = 15 (7,431 columns, N = 16) took 198 us
-  // against 60 + 117.
-  rc = dtype == BB_F64 ? launch_deriv<double>(ctx, t, K, 7, x, dr, ds, dt, st)
-                       : launch_deriv<float>(ctx, t, K, 7, x, dr, ds, dt, st);
-  if (rc) return rc;
-  return dtype == BB_F64 ? launch_lift<double>(ctx, t, K, 4, faces, lift, st)
-                         : launch_lift<float>(ctx, t, K, 4, faces, lift, st);
+  // against 60 + 117. The lift comes first where a gradient goes into the face columns' memory
+  // (Np = 4 Nfp at N = 9: the two have the same shape); each kernel itself reads a tile before it
+  // writes it.
+  const size_t size = dtype_size(dtype);
+  const size_t vol = (size_t)K * t->Np * size, fac = (size_t)K * 4 * t->Nfp * size;
+  auto into_faces = [&](const void* o) {
+    return (uintptr_t)o < (uintptr_t)faces + fac && (uintptr_t)faces < (uintptr_t)o + vol;
+  };
+  const bool lift_first = into_faces(dr) || into_faces(ds) || into_faces(dt);
+  for (int part = 0; part < 2; ++part) {
+    if ((part == 0) == lift_first)
+      rc = dtype == BB_F64 ? launch_lift<double>(ctx, t, K, 4, faces, lift, st)
+                           : launch_lift<float>(ctx, t, K, 4, faces, lift, st);
+    else
+      rc = dtype == BB_F64 ? launch_deriv<double>(ctx, t, K, 7, x, dr, ds, dt, st)
+                           : launch_deriv<float>(ctx, t, K, 7, x, dr, ds, dt, st);
+    if (rc) return rc;
+  }
+  return BB_OK;
 }
