@@ -238,11 +238,13 @@ __device__ __forceinline__ T deriv_row(int axis, int N, const T* x, int i, int j
 
 // Applies up to three derivative operators (mask bits r,s,t) to EPB element columns per
 // block iteration: stage the columns in shared memory, one thread per output coefficient.
+// Block `first` of `nblocks`.
 template <class T>
-__global__ void __launch_bounds__(256) deriv_kernel(DegTables tab, const uint32_t* __restrict__ gtab,
-                                                    int64_t K, int epb, int mask,
-                                                    const T* __restrict__ x, T* __restrict__ o0,
-                                                    T* __restrict__ o1, T* __restrict__ o2) {
+__device__ __forceinline__ void deriv_row_blocks(const DegTables& tab,
+                                                 const uint32_t* __restrict__ gtab, int64_t K,
+                                                 int epb, int mask, const T* __restrict__ x,
+                                                 T* __restrict__ o0, T* __restrict__ o1,
+                                                 T* __restrict__ o2, int first, int nblocks) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int N = tab.N, Np = tab.Np;
   T* sx = reinterpret_cast<T*>(smem);
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(256) deriv_kernel(DegTables tab, const uint32_
   const SmemTables st = load_tables(tab, gtab, stab);
   const int64_t nblk = (K + epb - 1) / epb;
   T* outs[3] = {o0, o1, o2};
-  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+  for (int64_t blk = first; blk < nblk; blk += nblocks) {
     const int64_t e0 = blk * epb;
     const int ne = (int)min64(epb, K - e0);
     __syncthreads();
@@ -267,18 +269,26 @@ __global__ void __launch_bounds__(256) deriv_kernel(DegTables tab, const uint32_
   }
 }
 
+template <class T>
+__global__ void __launch_bounds__(256) deriv_kernel(DegTables tab, const uint32_t* __restrict__ gtab,
+                                                    int64_t K, int epb, int mask,
+                                                    const T* __restrict__ x, T* __restrict__ o0,
+                                                    T* __restrict__ o1, T* __restrict__ o2) {
+  deriv_row_blocks(tab, gtab, K, epb, mask, x, o0, o1, o2, blockIdx.x, gridDim.x);
+}
+
 // Factored form of the same operators, D_a x(alpha) = 1/2 sum_b alpha_b w_a(alpha - e_b) with
 // w_a(beta) = x(beta + e_a) - x(beta + e_3) at degree N-1 (b over the four barycentric
 // indices; the reference's four terms per row, BernsteinDerivativeMatrix_3D.jl:96-216, are
 // exactly these). Per block: packed index tables in shared memory built once, then per tile
 // of EPB elements one pass forms w for every requested axis and one pass forms the outputs.
+// Block `first` of `nblocks`.
 template <class T>
-__global__ void __launch_bounds__(256) deriv_fact_kernel(DegTables tab,
-                                                         const uint32_t* __restrict__ gtab,
-                                                         int64_t K, int epb, int mask,
-                                                         const T* __restrict__ x,
-                                                         T* __restrict__ o0, T* __restrict__ o1,
-                                                         T* __restrict__ o2) {
+__device__ __forceinline__ void deriv_fact_blocks(const DegTables& tab,
+                                                  const uint32_t* __restrict__ gtab, int64_t K,
+                                                  int epb, int mask, const T* __restrict__ x,
+                                                  T* __restrict__ o0, T* __restrict__ o1,
+                                                  T* __restrict__ o2, int first, int nblocks) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int N = tab.N, Np = tab.Np, NPM1 = tab.NpM1, NW = NPM1 + 1;
   T* sx = reinterpret_cast<T*>(smem);                  // [epb][Np]
@@ -309,7 +319,7 @@ __global__ void __launch_bounds__(256) deriv_fact_kernel(DegTables tab,
   const uint64_t inv_m1 = 0xFFFFFFFFull / (uint64_t)NPM1 + 1ull;
   const uint64_t inv_np = 0xFFFFFFFFull / (uint64_t)Np + 1ull;
   const int64_t nblk = (K + epb - 1) / epb;
-  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+  for (int64_t blk = first; blk < nblk; blk += nblocks) {
     const int64_t e0 = blk * epb;
     const int ne = (int)min64(epb, K - e0);
     __syncthreads();
@@ -340,6 +350,16 @@ __global__ void __launch_bounds__(256) deriv_fact_kernel(DegTables tab,
       }
     }
   }
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) deriv_fact_kernel(DegTables tab,
+                                                         const uint32_t* __restrict__ gtab,
+                                                         int64_t K, int epb, int mask,
+                                                         const T* __restrict__ x,
+                                                         T* __restrict__ o0, T* __restrict__ o1,
+                                                         T* __restrict__ o2) {
+  deriv_fact_blocks(tab, gtab, K, epb, mask, x, o0, o1, o2, blockIdx.x, gridDim.x);
 }
 
 // -------------------------------------------------------------------------------------
@@ -373,11 +393,12 @@ static size_t lift_scalars(const DegTables& t, int nfaces, int epb) {
 // whole stack in shared memory (lift_stacks), then one pass sums the faces per coefficient. In
 // double the FP64 pipe bounds it (86 % of its rate at N = 7: 60,001 columns in 270 us, 417 with a
 // lift face by face that added every layer into the output, 4 (N+1) block barriers per tile).
+// Block `first` of `nblocks`.
 template <class T>
-__global__ void __launch_bounds__(256) lift_kernel(DegTables tab, const uint32_t* __restrict__ gtab,
-                                                   int64_t K, int epb,
-                                                   int nfaces, const T* __restrict__ x,
-                                                   T* __restrict__ out) {
+__device__ __forceinline__ void lift_blocks(const DegTables& tab,
+                                            const uint32_t* __restrict__ gtab, int64_t K, int epb,
+                                            int nfaces, const T* __restrict__ x,
+                                            T* __restrict__ out, int first, int nblocks) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int N = tab.N, Np = tab.Np, Nfp = tab.Nfp, gs = Np | 1;
   const int in_cols = nfaces * Nfp;
@@ -391,7 +412,7 @@ __global__ void __launch_bounds__(256) lift_kernel(DegTables tab, const uint32_t
   const uint4* gather = reinterpret_cast<const uint4*>(gtab + tab.o_gather);
   const FastDiv by_np(Np);
   const int64_t nblk = (K + epb - 1) / epb;
-  for (int64_t blk = blockIdx.x; blk < nblk; blk += gridDim.x) {
+  for (int64_t blk = first; blk < nblk; blk += nblocks) {
     const int64_t e0 = blk * epb;
     const int ne = (int)min64(epb, K - e0);
     __syncthreads();
@@ -404,6 +425,35 @@ __global__ void __launch_bounds__(256) lift_kernel(DegTables tab, const uint32_t
                                       : sG[(size_t)le * gs + n];
     }
   }
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) lift_kernel(DegTables tab, const uint32_t* __restrict__ gtab,
+                                                   int64_t K, int epb,
+                                                   int nfaces, const T* __restrict__ x,
+                                                   T* __restrict__ out) {
+  lift_blocks(tab, gtab, K, epb, nfaces, x, out, blockIdx.x, gridDim.x);
+}
+
+// Both operators side by side, for so few columns that all tiles of both are on the chip at once:
+// the first gd blocks do the gradient, the others the lift. Latency bounds such calls, not the
+// pipe (FP64, 384 columns, two launches / one: N = 1, 16.7 / 13.8 us; N = 9, 21.0 / 14.1; N = 17,
+// 101 / 58, with the per-row form's smaller tiles).
+template <class T>
+__global__ void __launch_bounds__(256) grad_lift_kernel(DegTables tab,
+                                                        const uint32_t* __restrict__ gtab,
+                                                        int64_t K, int epb_d, bool rows, int gd,
+                                                        const T* __restrict__ x,
+                                                        T* __restrict__ o0, T* __restrict__ o1,
+                                                        T* __restrict__ o2, int epb_l,
+                                                        const T* __restrict__ faces,
+                                                        T* __restrict__ out) {
+  if ((int)blockIdx.x >= gd)
+    lift_blocks(tab, gtab, K, epb_l, 4, faces, out, blockIdx.x - gd, gridDim.x - gd);
+  else if (rows)
+    deriv_row_blocks(tab, gtab, K, epb_d, 7, x, o0, o1, o2, blockIdx.x, gd);
+  else
+    deriv_fact_blocks(tab, gtab, K, epb_d, 7, x, o0, o1, o2, blockIdx.x, gd);
 }
 
 // 2D elevation (degree N -> N+1) or reduction (degree N -> N-1), one thread per output.
@@ -447,6 +497,40 @@ static int grid_for(bb_ctx* ctx, int64_t nblk, int per_sm) {
   return (int)(g < 1 ? 1 : g);
 }
 
+// Elements per block and shared memory of the gradient and lift kernels; tiles shrink until there
+// are two for every SM (or one element).
+struct OpTile {
+  int epb = 0;
+  size_t smem = 0;
+  bool rows = false;  // the per-row derivative form
+  int64_t blocks(int64_t K) const { return (K + epb - 1) / epb; }
+};
+template <class T>
+static OpTile deriv_tile(const bb_ctx* ctx, const DegTables& t, int64_t K) {
+  // factored form: tile of epb elements plus the w rows and the index tables
+  OpTile d;
+  for (d.epb = 16; d.epb >= 1; d.epb /= 2) {
+    d.smem = align16(sizeof(T) * ((size_t)d.epb * t.Np + 3 * (size_t)d.epb * (t.NpM1 + 1))) +
+             8 * (size_t)t.NpM1 + 8 * (size_t)t.Np + 4 * (size_t)t.Np;
+    if (d.smem <= 48 * 1024) return d;
+  }
+  d.rows = true;
+  for (d.epb = 8; d.epb > 1 && d.blocks(K) < 2 * ctx->num_sms;) d.epb /= 2;
+  d.smem = align16(sizeof(T) * (size_t)d.epb * t.Np) + 4 * (size_t)t.nwords;
+  return d;
+}
+template <class T>
+static OpTile lift_tile(const bb_ctx* ctx, const DegTables& t, int64_t K, int nfaces) {
+  // the most elements (up to 16) within 54 KB, four blocks per SM (FP64, N = 7: 284 / 270 / 312 us
+  // for 60,001 columns with 36 / 54 / 110 KB), that leave two blocks for every SM
+  OpTile l;
+  for (l.epb = 16; l.epb >= 1; l.epb /= 2) {
+    l.smem = align16(sizeof(T) * lift_scalars(t, nfaces, l.epb)) + 4 * (size_t)t.nwords;
+    if ((l.smem <= 54 * 1024 && l.blocks(K) >= 2 * ctx->num_sms) || l.epb == 1) break;
+  }
+  return l;
+}
+
 template <class T>
 static int launch_deriv(bb_ctx* ctx, const DegTables* t, int64_t K, int mask, const void* x,
                         void* o0, void* o1, void* o2, cudaStream_t st) {
@@ -454,33 +538,14 @@ static int launch_deriv(bb_ctx* ctx, const DegTables* t, int64_t K, int mask, co
     const int rc = bb_deriv_fast(ctx, t, K, mask, x, o0, o1, o2, st);
     if (rc >= 0) return rc;  // otherwise no specialised kernel for this degree or mask
   }
-  {
-    // factored kernel: tile of epb elements plus the w rows and the index tables
-    int epb = 16;
-    size_t smem = 0;
-    for (; epb >= 1; epb /= 2) {
-      smem = align16(sizeof(T) * ((size_t)epb * t->Np + 3 * (size_t)epb * (t->NpM1 + 1))) +
-             8 * (size_t)t->NpM1 + 8 * (size_t)t->Np + 4 * (size_t)t->Np;
-      if (smem <= 48 * 1024) break;
-    }
-    if (epb >= 1 && t->Np <= 65535) {
-      BB_CUDA(ctx, cudaFuncSetAttribute(deriv_fact_kernel<T>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      const int64_t nblk = (K + epb - 1) / epb;
-      deriv_fact_kernel<T><<<grid_for(ctx, nblk, 8), 256, smem, st>>>(
-          *t, t->d_words, K, epb, mask, (const T*)x, (T*)o0, (T*)o1, (T*)o2);
-      return bb_check_launch(ctx, "deriv_fact_kernel");
-    }
-  }
-  const int epb = 8;
-  const size_t smem = align16(sizeof(T) * (size_t)epb * t->Np) + 4 * (size_t)t->nwords;
-  if (smem > ctx->smem_optin) return bb_fail(ctx, BB_ERR_ARG, "degree too large for deriv tile");
-  BB_CUDA(ctx, cudaFuncSetAttribute(deriv_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-  const int64_t nblk = (K + epb - 1) / epb;
-  deriv_kernel<T><<<grid_for(ctx, nblk, 8), 256, smem, st>>>(
-      *t, t->d_words, K, epb, mask, (const T*)x, (T*)o0, (T*)o1, (T*)o2);
-  return bb_check_launch(ctx, "deriv_kernel");
+  const OpTile d = deriv_tile<T>(ctx, *t, K);
+  if (d.smem > ctx->smem_optin) return bb_fail(ctx, BB_ERR_ARG, "degree too large for deriv tile");
+  const auto kern = d.rows ? deriv_kernel<T> : deriv_fact_kernel<T>;
+  BB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)d.smem));
+  kern<<<grid_for(ctx, d.blocks(K), 8), 256, d.smem, st>>>(*t, t->d_words, K, d.epb, mask,
+                                                           (const T*)x, (T*)o0, (T*)o1, (T*)o2);
+  return bb_check_launch(ctx, d.rows ? "deriv_kernel" : "deriv_fact_kernel");
 }
 
 template <class T>
@@ -490,21 +555,30 @@ static int launch_lift(bb_ctx* ctx, const DegTables* t, int64_t K, int nfaces, c
     const int rc = bb_lift_fast(ctx, t, K, nfaces, x, out, st);
     if (rc >= 0) return rc;  // otherwise no specialised kernel for this degree
   }
-  // the most elements (up to 16) within 54 KB, four blocks per SM (FP64, N = 7: 284 / 270 / 312 us
-  // for 60,001 columns with 36 / 54 / 110 KB), that leave two blocks for every SM
-  int epb = 16;
-  size_t smem = 0;
-  for (; epb >= 1; epb /= 2) {
-    smem = align16(sizeof(T) * lift_scalars(*t, nfaces, epb)) + 4 * (size_t)t->nwords;
-    if ((smem <= 54 * 1024 && (K + epb - 1) / epb >= 2 * ctx->num_sms) || epb == 1) break;
-  }
-  if (smem > ctx->smem_optin) return bb_fail(ctx, BB_ERR_ARG, "degree too large for lift tile");
+  const OpTile l = lift_tile<T>(ctx, *t, K, nfaces);
+  if (l.smem > ctx->smem_optin) return bb_fail(ctx, BB_ERR_ARG, "degree too large for lift tile");
   BB_CUDA(ctx, cudaFuncSetAttribute(lift_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem));
-  const int64_t nblk = (K + epb - 1) / epb;
-  lift_kernel<T><<<grid_for(ctx, nblk, 8), 256, smem, st>>>(*t, t->d_words, K, epb, nfaces,
-                                                             (const T*)x, (T*)out);
+                                    (int)l.smem));
+  lift_kernel<T><<<grid_for(ctx, l.blocks(K), 8), 256, l.smem, st>>>(
+      *t, t->d_words, K, l.epb, nfaces, (const T*)x, (T*)out);
   return bb_check_launch(ctx, "lift_kernel");
+}
+
+// The table-driven gradient and lift in one launch; -1 where two are the better ones.
+template <class T>
+static int launch_grad_lift(bb_ctx* ctx, const DegTables* t, int64_t K, const void* x, void* dr,
+                            void* ds, void* dt, const void* faces, void* lift, cudaStream_t st) {
+  const OpTile d = deriv_tile<T>(ctx, *t, K), l = lift_tile<T>(ctx, *t, K, 4);
+  const size_t smem = d.smem > l.smem ? d.smem : l.smem;
+  const int64_t gd = d.blocks(K), gl = l.blocks(K);
+  const int64_t resident = min64(4, 228 * 1024 / (int64_t)(smem + 1024));
+  if (smem > ctx->smem_optin || gd + gl > resident * ctx->num_sms) return -1;
+  BB_CUDA(ctx, cudaFuncSetAttribute(grad_lift_kernel<T>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  grad_lift_kernel<T><<<(int)(gd + gl), 256, smem, st>>>(
+      *t, t->d_words, K, d.epb, d.rows, (int)gd, (const T*)x, (T*)dr, (T*)ds, (T*)dt, l.epb,
+      (const T*)faces, (T*)lift);
+  return bb_check_launch(ctx, "grad_lift_kernel");
 }
 
 static int check_common(bb_ctx* ctx, int N, int64_t K, int dtype) {
@@ -610,18 +684,24 @@ extern "C" int bb_fused_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const vo
   const DegTables* t = bb_tables(ctx, N);
   if (!t) return bb_fail(ctx, BB_ERR_NOMEM, "table allocation failed");
   cudaStream_t st = (cudaStream_t)stream;
-  // The gradient and lift calls back to back. One launch that read each input once was slower in
-  // both precisions: FP64 is bound by its pipe (60,001 columns, N = 7: 505 us fused, 192 + 270
-  // apart), FP32 has specialised kernels, and above N = 15 (7,431 columns, N = 16) took 198 us
-  // against 60 + 117. The lift comes first where a gradient goes into the face columns' memory
+  // The gradient and lift calls back to back, or side by side where all their tiles are on the
+  // chip at once. For many columns one launch that read each input once was slower in both
+  // precisions: FP64 is bound by its pipe (60,001 columns, N = 7: 505 us fused, 192 + 270 apart),
+  // FP32 has specialised kernels, and above N = 15 (7,431 columns, N = 16) took 198 us against
+  // 60 + 117. The lift comes first where a gradient goes into the face columns' memory
   // (Np = 4 Nfp at N = 9: the two have the same shape); each kernel itself reads a tile before it
   // writes it.
   const size_t size = dtype_size(dtype);
   const size_t vol = (size_t)K * t->Np * size, fac = (size_t)K * 4 * t->Nfp * size;
-  auto into_faces = [&](const void* o) {
-    return (uintptr_t)o < (uintptr_t)faces + fac && (uintptr_t)faces < (uintptr_t)o + vol;
+  auto into = [&](const void* in, size_t bytes, const void* o) {
+    return (uintptr_t)o < (uintptr_t)in + bytes && (uintptr_t)in < (uintptr_t)o + vol;
   };
-  const bool lift_first = into_faces(dr) || into_faces(ds) || into_faces(dt);
+  const bool lift_first = into(faces, fac, dr) || into(faces, fac, ds) || into(faces, fac, dt);
+  if ((dtype == BB_F64 || N > 15) && !lift_first && !into(x, vol, lift)) {
+    rc = dtype == BB_F64 ? launch_grad_lift<double>(ctx, t, K, x, dr, ds, dt, faces, lift, st)
+                         : launch_grad_lift<float>(ctx, t, K, x, dr, ds, dt, faces, lift, st);
+    if (rc >= 0) return rc;
+  }
   for (int part = 0; part < 2; ++part) {
     if ((part == 0) == lift_first)
       rc = dtype == BB_F64 ? launch_lift<double>(ctx, t, K, 4, faces, lift, st)

@@ -97,9 +97,9 @@ int bb_elevation_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const void* x, 
 int bb_reduction_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const void* x, void* out,
                        void* stream);
 
-/* Both operator passes: dr, ds, dt = D{r,s,t} x and lift = L faces, as two launches, the
- * gradient kernel and then the lift kernel, whose results equal bb_grad_apply and
- * bb_lift_apply bitwise. */
+/* Both operator passes: dr, ds, dt = D{r,s,t} x and lift = L faces, with results that equal
+ * bb_grad_apply's and bb_lift_apply's bitwise, in one launch where few columns (FP64, and FP32
+ * above N = 15) leave room on the GPU for both kernels side by side, else in two. */
 int bb_fused_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const void* x,
                    const void* faces, void* dr, void* ds, void* dt, void* lift, void* stream);
 
