@@ -6,6 +6,7 @@
 #include <array>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <new>
 #include <vector>
 
@@ -145,6 +146,43 @@ int stack_tile(bb_solver* s) {
   return best;
 }
 
+// The generic kernel's default tile: stack_tile's; where no tile holds whole stacks, one element.
+int generic_tile(bb_solver* s) {
+  const int e = stack_tile(s);
+  return e ? e : 1;
+}
+
+bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+// For the length of a call: the solver runs the generic kernel, on that kernel's own tile, if it
+// has a specialised one and one of the call's buffers is not on a 16-byte boundary, which that
+// one's bulk copies need. (The specialised kernel's tile is none to run the generic kernel on.
+// K = 4,374, two steps, specialised tile / default: Maxwell N = 3, 228 / 182 us, N = 9, 1,459 / 1,203,
+// N = 11, 3,132 / 2,345; wave N = 9, 649 / 572, N = 15, 3,589 / 2,603; but N = 5, 212 / 258.)
+struct KernelForBuffers {
+  bb_solver* s;
+  int fast, epb, threads;
+  size_t smem;
+  KernelForBuffers(bb_solver* s_, std::initializer_list<const void*> buffers)
+      : s(s_), fast(s_->fast), epb(s_->epb), threads(s_->threads), smem(s_->smem) {
+    bool aligned = aligned16(s->geo) && aligned16(s->conn);
+    for (const void* p : buffers) aligned = aligned && aligned16(p);
+    if (fast < 0 || aligned) return;
+    s->fast = -1;
+    s->epb = generic_tile(s);
+    s->threads = kThreads;
+    solver_layout(s, s->epb, &s->smem);
+  }
+  ~KernelForBuffers() {
+    s->fast = fast;
+    s->epb = epb;
+    s->threads = threads;
+    s->smem = smem;
+  }
+  KernelForBuffers(const KernelForBuffers&) = delete;
+  KernelForBuffers& operator=(const KernelForBuffers&) = delete;
+};
+
 // tb, te: the launch covers tiles [tb, te) of the solver's tile size (te = 0: all tiles).
 template <class T, int PHYS>
 int launch_stage_t(bb_solver* s, int mode, int stage, double dt, void* q, void* res, void* rhs,
@@ -220,14 +258,9 @@ int launch_fast(bb_solver* s, int mode, int stage, double dt, void* q, void* res
   return BB_OK;
 }
 
-bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
-
 int launch_stage(bb_solver* s, int mode, int stage, double dt, void* q, void* res, void* rhs,
                  const void* tin, void* tout, cudaStream_t st, int64_t tb = 0, int64_t te = 0) {
-  // the specialised kernels move tiles with 16-byte-aligned bulk copies and store q, res
-  // and rhs with 16-byte vector stores
-  if (s->fast >= 0 && aligned16(q) && (!res || aligned16(res)) && (!rhs || aligned16(rhs)) &&
-      aligned16(s->geo) && aligned16(s->conn))
+  if (s->fast >= 0)  // KernelForBuffers has looked at the buffers
     return launch_fast(s, mode, stage, dt, q, res, rhs, tin, tout, st, tb, te);
   if (s->physics == BB_WAVE)
     return s->dtype == BB_F64
@@ -341,17 +374,10 @@ extern "C" int bb_solver_create(bb_ctx* ctx, int physics, int N, int64_t K, int 
   s->geo = geo;
   s->tau = tau;
   s->tab = t;
-  // default tile: stack_tile's; where no tile holds whole stacks, one element
-  s->epb = stack_tile(s);
-  if (s->epb) solver_layout(s, s->epb, &s->smem);
-  if (!s->epb) {
-    size_t sm = 0;
-    if (solver_layout(s, 1, &sm) != BB_OK) {
-      delete s;
-      return bb_fail(ctx, BB_ERR_ARG, "degree %d does not fit in shared memory", N);
-    }
-    s->epb = 1;
-    s->smem = sm;
+  s->epb = generic_tile(s);
+  if (solver_layout(s, s->epb, &s->smem) != BB_OK) {
+    delete s;
+    return bb_fail(ctx, BB_ERR_ARG, "degree %d does not fit in shared memory", N);
   }
   if (dtype == BB_F32) {
     const int idx = bb_fast_find(N, physics, 0, 0);
@@ -444,7 +470,7 @@ extern "C" int bb_solver_set_kernel(bb_solver* s, int kind) {
   if (!s) return BB_ERR_ARG;
   if (kind != 0 && kind != 1) return bb_fail(s->ctx, BB_ERR_ARG, "kind must be 0 or 1");
   s->generic_only = kind;
-  if (kind == 1 && s->fast >= 0) return bb_solver_set_tile(s, s->epb, kThreads);
+  if (kind == 1 && s->fast >= 0) return bb_solver_set_tile(s, generic_tile(s), kThreads);
   if (kind == 0 && s->fast < 0 && s->dtype == BB_F32 && bb_fast_find(s->N, s->physics, 0, 0) >= 0)
     return bb_solver_set_tile(s, 0, 0);
   return BB_OK;
@@ -480,6 +506,7 @@ extern "C" int bb_rhs(bb_solver* s, const void* q, void* rhs, void* stream) {
   int rc = bb_set_device(s->ctx);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
+  const KernelForBuffers kernel(s, {q, rhs});
   rc = launch_stage(s, 0, 0, 0.0, const_cast<void*>(q), nullptr, rhs, nullptr, nullptr, st);
   if (rc) return rc;
   return check_status(s, st);
@@ -800,6 +827,7 @@ extern "C" int bb_lsrk_run(bb_solver* s, double dt, int nsteps, void* q, void* r
   if (rc) return rc;
   if (nsteps == 0) return BB_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  const KernelForBuffers kernel(s, {q, res});
   // traces of the incoming state; stage kernels then keep them current
   rc = launch_extract(s, q, s->trace[0], st);
   if (rc) return rc;
@@ -875,6 +903,7 @@ extern "C" int bb_lsrk_run_host(bb_solver* s, double dt, int nsteps, const void*
     BB_CUDA(s->ctx, cudaMemcpyAsync(q_host_out, q_dev, bytes, cudaMemcpyDeviceToHost, st));
     return BB_OK;
   }
+  const KernelForBuffers kernel(s, {q_dev, res_dev});
   rc = ensure_host_streams(s);
   if (rc) return rc;
   rc = build_host_plan(s);

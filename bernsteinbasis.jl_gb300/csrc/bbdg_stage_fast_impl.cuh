@@ -1209,14 +1209,12 @@ int FastKernel<N, PHYS, EPB, TPE>::launch(const FastLaunch& fl, const FastStageP
                                           cudaStream_t st) {
   constexpr int NP = FastLayout<N, PHYS, EPB, TPE>::NP;
   FastStageParams P = P0;
-  // widest copy (floats) that every field row of every tile is aligned for: rows start at
-  // multiples of EPB NP and of K NP floats
-  const uintptr_t base = (uintptr_t)P.q | (uintptr_t)P.res;
-  auto fits = [&](int v) {
-    return base % (4 * v) == 0 && (EPB * NP) % v == 0 && (P.K * NP) % v == 0;
-  };
+  // widest copy (floats) that every field row of every tile is aligned for: the callers pass
+  // 16-byte-aligned buffers, and rows start at multiples of EPB NP and of K NP floats
+  if ((((uintptr_t)P.q | (uintptr_t)P.res | (uintptr_t)P.geo | (uintptr_t)P.conn) & 15) != 0)
+    return BB_ERR_ARG;
+  auto fits = [&](int v) { return (EPB * NP) % v == 0 && (P.K * NP) % v == 0; };
   P.vec = fits(4) ? 4 : fits(2) ? 2 : 1;
-  if (NP % 4 == 0 && P.vec != 4) return BB_ERR_ARG;  // the callers pass 16-byte-aligned buffers
   if constexpr ((EPB * NP) % 4 == 0)
     if (P.vec == 4 && P.K % EPB == 0)
       return launch_fast_any<N, PHYS, EPB, TPE, false>(fl, P, st);
