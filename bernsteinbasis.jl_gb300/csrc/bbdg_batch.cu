@@ -41,8 +41,10 @@ struct BatchDesc {
   int physics;
 };
 
-template <class T>
-__global__ void __launch_bounds__(kBatchThreads, 3)
+// THREADS 256, or 512 for tiles of which one fills an SM's shared memory (as the single solver's
+// stage kernel).
+template <class T, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kBatchThreads ? 3 : 1)
     batch_stage_kernel(const BatchDesc<T>* __restrict__ descs, int nprob, int64_t total,
                        unsigned long long* counter, int par, T rkA, T rkB) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -106,14 +108,22 @@ struct bb_batch {
   // persistent launch gives each block its tiles up front, so a block that another problem's
   // kernel keeps off its SM ends late by all of its tiles
   std::vector<int> small, large;
-  int nfast = 0, ngeneric = 0;
+  // generic problems: one launch per stage for those whose tiles leave room for two blocks and more
+  // on an SM, and one for those whose tile fills it. In one launch, whose shared memory is that of
+  // its largest tile, one problem of the second kind would leave each SM one block of every other
+  // problem too (FP64, two steps of Maxwell N = 11, K = 384, beside waves N = 5 and 7 and a Maxwell
+  // N = 5 of some 10,000 elements: one launch 8,287 us, two 6,733; Maxwell N = 12 alone, 256 threads
+  // 2,225 us, 512 2,075).
+  struct Lane {
+    int first = 0, count = 0;  // descriptors
+    int64_t total = 0;         // work items
+    size_t smem = 0;
+    int threads = kBatchThreads, grid = 0;
+  } lane[2];
   std::vector<void*> trace;      // 2 per problem
   void* d_desc = nullptr;
-  unsigned long long* d_counter = nullptr;  // 5 stage counters
+  unsigned long long* d_counter = nullptr;  // 5 stage counters per lane
   int* d_status = nullptr;
-  int64_t total = 0;
-  size_t smem = 0;
-  int grid = 0;
   bool dirty = true;             // descriptors need rebuilding
   cudaStream_t cap = nullptr;
   cudaStream_t side[kSideStreams] = {};
@@ -144,13 +154,18 @@ void drop_batch_graphs(bb_batch* b) {
 }
 
 template <class T>
+auto batch_kernel(int threads) {
+  return threads == kBatchThreads ? batch_stage_kernel<T, kBatchThreads>
+                                  : batch_stage_kernel<T, 2 * kBatchThreads>;
+}
+
+template <class T>
 int build_desc(bb_batch* b) {
   bb_ctx* ctx = b->ctx;
   const int np = (int)b->probs.size();
   auto a16 = [](const void* x) { return ((uintptr_t)x & 15) == 0; };
   b->fast.assign(np, -1);
   b->fast_tables.assign(np, nullptr);
-  b->nfast = b->ngeneric = 0;
   b->small.clear();
   b->large.clear();
   for (int p = 0; p < np; ++p) {
@@ -165,7 +180,6 @@ int build_desc(bb_batch* b) {
     if (b->fast[p] >= 0) {
       b->fast_tables[p] = bb_fast_tables(ctx, b->fast[p]);
       if (!b->fast_tables[p]) return bb_fail(ctx, BB_ERR_NOMEM, "table allocation failed");
-      ++b->nfast;
       int e = 0, th = 0;
       size_t sm = 0;
       bb_fast_variant_info(b->fast[p], &e, &th, &sm);
@@ -174,54 +188,63 @@ int build_desc(bb_batch* b) {
     }
   }
   std::vector<BatchDesc<T>> h;
-  int64_t begin = 0;
-  size_t smem = 0;
-  for (int p = 0; p < np; ++p) {
-    if (b->fast[p] >= 0) continue;
-    const bb_batch_problem& pr = b->probs[p];
-    const DegTables* t = b->tabs[p];
-    h.push_back(BatchDesc<T>{});  // every field zero (the degree tables' own defaults)
-    BatchDesc<T>& d = h.back();
-    d.P.tab = *t;
-    d.P.gtab = t->d_words;
-    d.P.K = pr.K;
-    d.P.epb = b->epb[p];
-    d.P.mode = 1;
-    d.P.dt = T(pr.dt);
-    d.P.tau = T(pr.tau);
-    d.P.q = (T*)pr.q;
-    d.P.res = (T*)pr.res;
-    d.P.geo = (const T*)pr.geo;
-    d.P.conn = pr.conn;
-    d.P.status = b->d_status;
-    d.trace[0] = (T*)b->trace[2 * p];
-    d.trace[1] = (T*)b->trace[2 * p + 1];
-    d.tile_begin = begin;
-    d.physics = pr.physics;
-    begin += (pr.K + b->epb[p] - 1) / b->epb[p];
-    const int nf = physics_nf(pr.physics);
-    const TileLayout L = tile_layout_for(pr.N, nf, nf, sizeof(T), t->nwords, b->epb[p]);
-    smem = std::max(smem, L.total);
+  for (int ln = 0; ln < 2; ++ln) {
+    bb_batch::Lane& lane = b->lane[ln];
+    lane = bb_batch::Lane{};
+    lane.first = (int)h.size();
+    for (int p = 0; p < np; ++p) {
+      if (b->fast[p] >= 0) continue;
+      const bb_batch_problem& pr = b->probs[p];
+      const DegTables* t = b->tabs[p];
+      const int nf = physics_nf(pr.physics);
+      const TileLayout L = tile_layout_for(pr.N, nf, nf, sizeof(T), t->nwords, b->epb[p]);
+      if (ln != (2 * (L.total + 1024) > 228 * 1024)) continue;
+      h.push_back(BatchDesc<T>{});  // every field zero (the degree tables' own defaults)
+      BatchDesc<T>& d = h.back();
+      d.P.tab = *t;
+      d.P.gtab = t->d_words;
+      d.P.K = pr.K;
+      d.P.epb = b->epb[p];
+      d.P.mode = 1;
+      d.P.dt = T(pr.dt);
+      d.P.tau = T(pr.tau);
+      d.P.q = (T*)pr.q;
+      d.P.res = (T*)pr.res;
+      d.P.geo = (const T*)pr.geo;
+      d.P.conn = pr.conn;
+      d.P.status = b->d_status;
+      d.trace[0] = (T*)b->trace[2 * p];
+      d.trace[1] = (T*)b->trace[2 * p + 1];
+      d.tile_begin = lane.total;
+      d.physics = pr.physics;
+      lane.total += (pr.K + b->epb[p] - 1) / b->epb[p];
+      lane.smem = std::max(lane.smem, L.total);
+    }
+    lane.count = (int)h.size() - lane.first;
   }
-  b->ngeneric = (int)h.size();
-  b->total = begin;
-  b->smem = smem;
   if (h.empty()) {
     b->dirty = false;
     return BB_OK;
   }
-  if (smem > ctx->smem_optin) return bb_fail(ctx, BB_ERR_ARG, "batch tiles exceed shared memory");
   if (!b->d_desc) {
     BB_CUDA(ctx, cudaMalloc(&b->d_desc, sizeof(BatchDesc<T>) * np));
   }
   BB_CUDA(ctx, upload_bytes(ctx->device, b->d_desc, h.data(), sizeof(BatchDesc<T>) * h.size()));
-  BB_CUDA(ctx, cudaFuncSetAttribute(batch_stage_kernel<T>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int per_sm = 0;
-  BB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_stage_kernel<T>,
-                                                             kBatchThreads, smem));
-  if (per_sm < 1) return bb_fail(ctx, BB_ERR_ARG, "batch tile does not fit on an SM");
-  b->grid = (int)std::min<int64_t>((int64_t)per_sm * ctx->num_sms, std::max<int64_t>(b->total, 1));
+  for (int ln = 0; ln < 2; ++ln) {
+    bb_batch::Lane& lane = b->lane[ln];
+    if (lane.count == 0) continue;
+    if (lane.smem > ctx->smem_optin)
+      return bb_fail(ctx, BB_ERR_ARG, "batch tiles exceed shared memory");
+    lane.threads = (ln + 1) * kBatchThreads;
+    const auto kern = batch_kernel<T>(lane.threads);
+    BB_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)lane.smem));
+    int per_sm = 0;
+    BB_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, lane.threads,
+                                                               lane.smem));
+    if (per_sm < 1) return bb_fail(ctx, BB_ERR_ARG, "batch tile does not fit on an SM");
+    lane.grid = (int)std::min<int64_t>((int64_t)per_sm * ctx->num_sms, lane.total);
+  }
   b->dirty = false;
   return BB_OK;
 }
@@ -273,15 +296,18 @@ int enqueue_batch_step(bb_batch* b, int par, cudaStream_t st) {
       }
     }
   }
-  if (b->ngeneric > 0) {
-    BB_CUDA(ctx, cudaMemsetAsync(b->d_counter, 0, 5 * sizeof(unsigned long long), st));
-    for (int s = 0; s < 5; ++s) {
-      batch_stage_kernel<T><<<b->grid, kBatchThreads, b->smem, st>>>(
-          (const BatchDesc<T>*)b->d_desc, b->ngeneric, b->total, b->d_counter + s,
-          (par + s) & 1, T(kA[s]), T(kB[s]));
-      int rc = bb_check_launch(ctx, "batch_stage_kernel");
-      if (rc) return rc;
-    }
+  if (b->lane[0].count + b->lane[1].count > 0) {
+    BB_CUDA(ctx, cudaMemsetAsync(b->d_counter, 0, 10 * sizeof(unsigned long long), st));
+    for (int s = 0; s < 5; ++s)
+      for (int ln = 0; ln < 2; ++ln) {
+        const bb_batch::Lane& lane = b->lane[ln];
+        if (lane.count == 0) continue;
+        batch_kernel<T>(lane.threads)<<<lane.grid, lane.threads, lane.smem, st>>>(
+            (const BatchDesc<T>*)b->d_desc + lane.first, lane.count, lane.total,
+            b->d_counter + 5 * ln + s, (par + s) & 1, T(kA[s]), T(kB[s]));
+        int rc = bb_check_launch(ctx, "batch_stage_kernel");
+        if (rc) return rc;
+      }
   }
   for (int i = 0; i < nside; ++i) {  // join
     BB_CUDA(ctx, cudaEventRecord(b->join_ev[i], b->side[i]));
@@ -414,7 +440,7 @@ extern "C" int bb_batch_create(bb_ctx* ctx, int nprob, const bb_batch_problem* p
       b->trace.push_back(ptr);
     }
   }
-  if (cudaMalloc(&b->d_counter, 5 * sizeof(unsigned long long)) != cudaSuccess ||
+  if (cudaMalloc(&b->d_counter, 10 * sizeof(unsigned long long)) != cudaSuccess ||
       cudaMalloc(&b->d_status, sizeof(int)) != cudaSuccess ||
       cudaMemset(b->d_status, 0, sizeof(int)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking) != cudaSuccess ||
