@@ -128,7 +128,8 @@ struct Lift4 {
 };
 
 template <int N>
-__global__ void __launch_bounds__(32) lift4_kernel(int64_t K, const float* __restrict__ x,
+__global__ void __launch_bounds__(32) lift4_kernel(int64_t K, const uint4* __restrict__ gather,
+                                                   const float* __restrict__ x,
                                                    float* __restrict__ out, int* status,
                                                    uint32_t wait_iters) {
   using L = Lift4<N>;
@@ -139,15 +140,24 @@ __global__ void __launch_bounds__(32) lift4_kernel(int64_t K, const float* __res
   float* sG = reinterpret_cast<float*>(smem + L::G_B);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + L::BAR_B);
   const int t = threadIdx.x;
-  // stack positions of coefficient n on faces f0 (i,k,j), f1 (j,k,l), f2 (j,k,i), f3 (i,j,k)
-  auto positions = [](int n) {
-    int m = n, k = 0, j = 0;
-    while (m >= (N - k + 1) * (N - k + 2) / 2) m -= (N - k + 1) * (N - k + 2) / 2, ++k;
-    while (m >= N - k - j + 1) m -= N - k - j + 1, ++j;
-    const int i = m, l = N - i - j - k;
-    auto at = [](int q) { return (uint32_t)(L::SLOTS ? lift_slot_at<N>(q) : q); };
-    return make_uint2(at(lf_ijk(N, i, k, j)) | (at(lf_ijk(N, j, k, l)) << 16),
-                      at(lf_ijk(N, j, k, i)) | (at(n) << 16));
+  // stack positions of coefficient n on faces f0 (i,k,j), f1 (j,k,l), f2 (j,k,i), f3 (i,j,k): from
+  // the degree's gather table, or decoded where that takes less than a load (up to degree 4; 384
+  // columns, table / decoded: N = 4, 2.5 / 2.3 us, N = 9, 6.6 / 7.6, N = 12, 7.6 / 11.5, N = 15,
+  // 11.1 / 18.6)
+  auto positions = [=](int n) {
+    if constexpr (N <= 4) {
+      int m = n, k = 0, j = 0;
+      while (m >= (N - k + 1) * (N - k + 2) / 2) m -= (N - k + 1) * (N - k + 2) / 2, ++k;
+      while (m >= N - k - j + 1) m -= N - k - j + 1, ++j;
+      const int i = m, l = N - i - j - k;
+      return make_uint2(lf_ijk(N, i, k, j) | (lf_ijk(N, j, k, l) << 16), lf_ijk(N, j, k, i) | (n << 16));
+    } else {
+      const uint4 ga = __ldg(gather + n);
+      if constexpr (!L::SLOTS) return make_uint2(ga.z, ga.w);
+      auto at = [](uint32_t q) { return (uint32_t)lift_slot_at<N>((int)q); };
+      return make_uint2(at(ga.z & 0xffffu) | (at(ga.z >> 16) << 16),
+                        at(ga.w & 0xffffu) | (at(ga.w >> 16) << 16));
+    }
   };
   auto pack = [](uint2 p) {  // f0, f1, f2, 10 bits each (f3 is n itself in volume order)
     return (p.x & 0xffffu) | ((p.x >> 16) << 10) | ((p.y & 0xffffu) << 20);
@@ -336,7 +346,8 @@ __global__ void __launch_bounds__(32) lift4_kernel(int64_t K, const float* __res
 }
 
 template <int N>
-int launch_lift4(bb_ctx* ctx, int64_t K, const void* x, void* out, cudaStream_t st) {
+int launch_lift4(bb_ctx* ctx, const DegTables* t, int64_t K, const void* x, void* out,
+                 cudaStream_t st) {
   using L = Lift4<N>;
   auto kern = lift4_kernel<N>;
   int* status = bb_ctx_status_word(ctx);
@@ -347,7 +358,8 @@ int launch_lift4(bb_ctx* ctx, int64_t K, const void* x, void* out, cudaStream_t 
   if (per_sm < 1) return bb_fail(ctx, BB_ERR_ARG, "lift tile does not fit");
   const int64_t ntile = (K + L::EPW - 1) / L::EPW;
   const int grid = (int)std::min<int64_t>(ntile, (int64_t)per_sm * ctx->num_sms);
-  kern<<<grid, 32, L::SMEM, st>>>(K, (const float*)x, (float*)out, status, ctx->wait_iters);
+  kern<<<grid, 32, L::SMEM, st>>>(K, reinterpret_cast<const uint4*>(t->d_words + t->o_gather),
+                                  (const float*)x, (float*)out, status, ctx->wait_iters);
   return bb_check_launch(ctx, "lift4_kernel");
 }
 
