@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "bbdg_gemm.cuh"
@@ -152,19 +153,33 @@ __global__ void transpose_bf16_kernel(const __nv_bfloat16* __restrict__ in, int6
   }
 }
 
-// Elements per block of the closure's gather (features) and update (apply) kernels. The position
+// Elements per block (E) of the closure's gather (features) and update (apply) kernels. The position
 // (field, face, node) of a value is decoded once for all of them, and their loads are in flight
 // together. One element per block with the decoding in 64 bits kept the ALUs busy for 75 us
 // (features) and 29 us (apply) at degree 5, six fields, 24,576 elements; now 34 us and 13 us.
 // Features by 4 instead of 8 elements: 44 against 40 us; apply by 8 instead of 4: 14.6 against 13.
-constexpr int kClosureElems = 8;
+// Few elements are spread over the SMs instead (ClosureGrid): features of 200 elements in FP64, degree
+// 7, four fields, 7.1 us by eights and 2.9 spread; apply of 48, 2.9 and 1.9.
+constexpr int kFeatureElems = 8;
 constexpr int kApplyElems = 4;
+struct ClosureGrid {
+  int per_block;  // elements: at most `most`, fewer as long as there are less than `want` blocks
+  int threads;    // no more warps than an element has values
+  dim3 grid;      // x: elements; y: parts of an element's values, where x alone is less than `want`
+  ClosureGrid(int64_t K, int values, int most, int64_t want) : per_block(most) {
+    while (per_block > 1 && (K + per_block - 1) / per_block < want) per_block /= 2;
+    threads = std::min(256, std::max(64, (values + 31) / 32 * 32));
+    const int64_t x = (K + per_block - 1) / per_block;
+    grid = dim3((unsigned)std::min<int64_t>(x, INT32_MAX),
+                (unsigned)std::min<int64_t>((values + threads - 1) / threads, (want + x - 1) / x));
+  }
+};
 
 // Closure features of element e (nf fields, degree N), scaled and rounded to BF16:
 //   [fld][p]        own coefficients, p < Np
 //   [f][fld][a]     the neighbour's coefficients on the shared face f, face node a < Nfp, in
 //                   this element's face ordering (the exterior trace the flux sees)
-template <class T>
+template <class T, int E>
 __global__ void closure_features_kernel(const uint32_t* __restrict__ gtab, int o_fvol,
                                         int o_fperm, int N, int64_t K, int nf,
                                         const int32_t* __restrict__ conn,
@@ -174,12 +189,12 @@ __global__ void closure_features_kernel(const uint32_t* __restrict__ gtab, int o
   const int nown = nf * Np, nin = nown + 4 * nf * Nfp;
   const uint16_t* fvol = reinterpret_cast<const uint16_t*>(gtab + o_fvol);
   const uint16_t* fperm = reinterpret_cast<const uint16_t*>(gtab + o_fperm);
-  const int64_t e0 = (int64_t)blockIdx.x * kClosureElems;
-  const int ne = (int)(K - e0 < kClosureElems ? K - e0 : kClosureElems);
+  const int64_t e0 = (int64_t)blockIdx.x * E;
+  const int ne = (int)(K - e0 < E ? K - e0 : E);
   // per element and face: the neighbour (-1: corrupt connectivity), where its face nodes and the
   // node permutation of the orientation start
-  __shared__ int s_nbr[kClosureElems][4], s_vol[kClosureElems][4], s_perm[kClosureElems][4];
-  if (threadIdx.x < 4 * kClosureElems) {
+  __shared__ int s_nbr[E][4], s_vol[E][4], s_perm[E][4];
+  if (threadIdx.x < 4 * E) {
     const int u = threadIdx.x >> 2, f = threadIdx.x & 3;
     const int32_t c = u < ne ? __ldg(conn + (e0 + u) * 4 + f) : 0;
     const int64_t nbr = (int64_t)((uint32_t)c >> 5);
@@ -191,53 +206,53 @@ __global__ void closure_features_kernel(const uint32_t* __restrict__ gtab, int o
     s_perm[u][f] = bad ? 0 : o * Nfp;
   }
   __syncthreads();
-  for (int t = threadIdx.x; t < nin; t += blockDim.x) {
-    float val[kClosureElems];
+  for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < nin; t += gridDim.y * blockDim.x) {
+    float val[E];
     if (t < nown) {
       const int fld = t / Np, p = t - fld * Np;
       const T* src = q + ((int64_t)fld * K + e0) * Np + p;
 #pragma unroll
-      for (int u = 0; u < kClosureElems; ++u) val[u] = u < ne ? (float)src[u * Np] : 0.0f;
+      for (int u = 0; u < E; ++u) val[u] = u < ne ? (float)src[u * Np] : 0.0f;
     } else {
       const int u0 = t - nown;
       const int f = u0 / (nf * Nfp), rest = u0 - f * nf * Nfp;
       const int fld = rest / Nfp, a = rest - fld * Nfp;
       const T* src = q + (int64_t)fld * K * Np;
-      int vP[kClosureElems];
+      int vP[E];
 #pragma unroll
-      for (int u = 0; u < kClosureElems; ++u)
+      for (int u = 0; u < E; ++u)
         vP[u] = __ldg(fvol + s_vol[u][f] + __ldg(fperm + s_perm[u][f] + a));
 #pragma unroll
-      for (int u = 0; u < kClosureElems; ++u) {
+      for (int u = 0; u < E; ++u) {
         const int nbr = s_nbr[u][f];
         val[u] = nbr < 0 ? 0.0f : (float)src[(int64_t)nbr * Np + vP[u]];
       }
     }
 #pragma unroll
-    for (int u = 0; u < kClosureElems; ++u)
+    for (int u = 0; u < E; ++u)
       if (u < ne) X[(e0 + u) * nin + t] = __float2bfloat16_rn(val[u] * scale);
   }
 }
 
 // q[fld][e][p] += alpha * Y[e][fld * Np + p]
-template <class T>
+template <class T, int E>
 __global__ void closure_apply_kernel(int Np, int64_t K, int nf, float alpha,
                                      const float* __restrict__ Y, T* __restrict__ q) {
   const int nw = nf * Np;
-  const int64_t e0 = (int64_t)blockIdx.x * kApplyElems;
-  const int ne = (int)(K - e0 < kApplyElems ? K - e0 : kApplyElems);
-  for (int t = threadIdx.x; t < nw; t += blockDim.x) {
+  const int64_t e0 = (int64_t)blockIdx.x * E;
+  const int ne = (int)(K - e0 < E ? K - e0 : E);
+  for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < nw; t += gridDim.y * blockDim.x) {
     const int fld = t / Np, p = t - fld * Np;
     T* dst = q + ((int64_t)fld * K + e0) * Np + p;
     const float* src = Y + e0 * nw + t;
-    float y[kApplyElems], v[kApplyElems];
+    float y[E], v[E];
 #pragma unroll
-    for (int u = 0; u < kApplyElems; ++u) {
+    for (int u = 0; u < E; ++u) {
       y[u] = u < ne ? src[(int64_t)u * nw] : 0.0f;
       v[u] = u < ne ? (float)dst[(int64_t)u * Np] : 0.0f;
     }
 #pragma unroll
-    for (int u = 0; u < kApplyElems; ++u)
+    for (int u = 0; u < E; ++u)
       if (u < ne) dst[(int64_t)u * Np] = (T)(v[u] + alpha * y[u]);
   }
 }
@@ -535,15 +550,21 @@ extern "C" int bb_closure_features(bb_ctx* ctx, int N, int64_t K, int nf, const 
   int* status = bb_ctx_status_word(ctx);
   if (!status) return bb_fail(ctx, BB_ERR_NOMEM, "status word allocation failed");
   cudaStream_t st = (cudaStream_t)stream;
-  const int64_t grid = (K + kClosureElems - 1) / kClosureElems;
-  if (dtype == BB_F64)
-    closure_features_kernel<double><<<(unsigned)grid, 256, 0, st>>>(t->d_words, t->o_fvol, t->o_fperm, N, K,
-                                                          nf, conn, (const double*)q, scale,
-                                                          (__nv_bfloat16*)X, status);
-  else
-    closure_features_kernel<float><<<(unsigned)grid, 256, 0, st>>>(t->d_words, t->o_fvol, t->o_fperm, N, K,
-                                                         nf, conn, (const float*)q, scale,
-                                                         (__nv_bfloat16*)X, status);
+  const ClosureGrid g(K, nf * (np3(N) + 4 * np2(N)), kFeatureElems, 4 * ctx->num_sms);
+  const int per_block = g.per_block;
+  auto go = [&](auto kern, auto* qt) {
+    kern<<<g.grid, g.threads, 0, st>>>(t->d_words, t->o_fvol, t->o_fperm, N, K, nf, conn, qt, scale,
+                                       (__nv_bfloat16*)X, status);
+  };
+  auto pick = [&](auto* qt) {
+    using T = std::remove_const_t<std::remove_pointer_t<decltype(qt)>>;
+    if (per_block == 8) go(closure_features_kernel<T, 8>, qt);
+    else if (per_block == 4) go(closure_features_kernel<T, 4>, qt);
+    else if (per_block == 2) go(closure_features_kernel<T, 2>, qt);
+    else go(closure_features_kernel<T, 1>, qt);
+  };
+  if (dtype == BB_F64) pick((const double*)q);
+  else pick((const float*)q);
   rc = bb_check_launch(ctx, "closure_features_kernel");
   if (rc || !XT) return rc;
   const int nin = nf * np3(N) + 4 * nf * np2(N);
@@ -559,11 +580,20 @@ extern "C" int bb_closure_apply(bb_ctx* ctx, int N, int64_t K, int nf, int dtype
   if (rc) return rc;
   if (K == 0) return BB_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const int64_t grid = (K + kApplyElems - 1) / kApplyElems;
-  if (grid > INT32_MAX) return bb_fail(ctx, BB_ERR_ARG, "bad argument to bb_closure_apply");
-  if (dtype == BB_F64)
-    closure_apply_kernel<double><<<(unsigned)grid, 256, 0, st>>>(np3(N), K, nf, alpha, Y, (double*)q);
-  else
-    closure_apply_kernel<float><<<(unsigned)grid, 256, 0, st>>>(np3(N), K, nf, alpha, Y, (float*)q);
+  // in double the conversions bound few elements, so they are spread wider
+  const ClosureGrid g(K, nf * np3(N), kApplyElems, (dtype == BB_F64 ? 4 : 1) * ctx->num_sms);
+  const int per_block = g.per_block;
+  if (K / per_block >= INT32_MAX) return bb_fail(ctx, BB_ERR_ARG, "bad argument to bb_closure_apply");
+  auto go = [&](auto kern, auto* qt) {
+    kern<<<g.grid, g.threads, 0, st>>>(np3(N), K, nf, alpha, Y, qt);
+  };
+  auto pick = [&](auto* qt) {
+    using T = std::remove_pointer_t<decltype(qt)>;
+    if (per_block == 4) go(closure_apply_kernel<T, 4>, qt);
+    else if (per_block == 2) go(closure_apply_kernel<T, 2>, qt);
+    else go(closure_apply_kernel<T, 1>, qt);
+  };
+  if (dtype == BB_F64) pick((double*)q);
+  else pick((float*)q);
   return bb_check_launch(ctx, "closure_apply_kernel");
 }
