@@ -219,10 +219,9 @@ __device__ __forceinline__ void epi_rows(const GemmEpilogue& ep, float* T, int r
         }
         x4 = make_float4(x[0], x[1], x[2], x[3]);
         if (F & kCf) *reinterpret_cast<float4*>(ep.Cf + off) = x4;
-        if (F & kCfAdd) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) atomicAdd(ep.Cf + off + j, x[j]);
-        }
+        // one vector reduction (element by element atomic) in place of four that each touch every
+        // fourth float of the same segments
+        if (F & kCfAdd) atomicAdd(reinterpret_cast<float4*>(ep.Cf + off), x4);
         if (F & kCb) st_bf16x4(ep.Cb + off, x4);
       } else {
 #pragma unroll
