@@ -701,15 +701,28 @@ extern "C" int bb_fused_apply(bb_ctx* ctx, int N, int64_t K, int dtype, const vo
     rc = dtype == BB_F64 ? launch_grad_lift<double>(ctx, t, K, x, dr, ds, dt, faces, lift, st)
                          : launch_grad_lift<float>(ctx, t, K, x, dr, ds, dt, faces, lift, st);
     if (rc >= 0) return rc;
+    rc = BB_OK;
   }
-  for (int part = 0; part < 2; ++part) {
+  // A gradient into the face columns and the lift into x: no order of the two will do, so the lift
+  // goes through memory of its own.
+  void* const out = lift;
+  if (lift_first && into(x, vol, lift) && cudaMallocAsync(&lift, vol, st) != cudaSuccess) {
+    cudaGetLastError();
+    return bb_fail(ctx, BB_ERR_NOMEM, "allocation for exchanged buffers failed");
+  }
+  for (int part = 0; part < 2 && rc == BB_OK; ++part) {
     if ((part == 0) == lift_first)
       rc = dtype == BB_F64 ? launch_lift<double>(ctx, t, K, 4, faces, lift, st)
                            : launch_lift<float>(ctx, t, K, 4, faces, lift, st);
     else
       rc = dtype == BB_F64 ? launch_deriv<double>(ctx, t, K, 7, x, dr, ds, dt, st)
                            : launch_deriv<float>(ctx, t, K, 7, x, dr, ds, dt, st);
-    if (rc) return rc;
   }
-  return BB_OK;
+  if (lift != out) {
+    cudaError_t e = cudaSuccess;
+    if (rc == BB_OK) e = cudaMemcpyAsync(out, lift, vol, cudaMemcpyDeviceToDevice, st);
+    const cudaError_t f = cudaFreeAsync(lift, st);
+    if (rc == BB_OK) BB_CUDA(ctx, e != cudaSuccess ? e : f);
+  }
+  return rc;
 }
