@@ -159,19 +159,23 @@ __global__ void transpose_bf16_kernel(const __nv_bfloat16* __restrict__ in, int6
 // (features) and 29 us (apply) at degree 5, six fields, 24,576 elements; now 34 us and 13 us.
 // Features by 4 instead of 8 elements: 44 against 40 us; apply by 8 instead of 4: 14.6 against 13.
 // Few elements are spread over the SMs instead (ClosureGrid): features of 200 elements in FP64, degree
-// 7, four fields, 7.1 us by eights and 2.9 spread; apply of 48, 2.9 and 1.9.
+// 7, four fields, 7.1 us by eights and 2.9 spread; apply of 48, 2.9 and 1.9. The update's values are
+// cheap to decode, so its blocks share out an element's values as long as there are less than 16 for
+// every SM, which makes a last round with few blocks shorter (six fields, degree 10, whole / shared
+// out: 1,296 elements in FP64 11.9 / 9.9 us, 3,072 24.2 / 20.7; 3,072 in FP32 8.8 / 7.0. Features lose
+// as often as they gain by it: FP64, degree 7, 384 elements 4.6 / 5.0, 3,072 14.0 / 12.0).
 constexpr int kFeatureElems = 8;
 constexpr int kApplyElems = 4;
 struct ClosureGrid {
   int per_block;  // elements: at most `most`, fewer as long as there are less than `want` blocks
   int threads;    // no more warps than an element has values
-  dim3 grid;      // x: elements; y: parts of an element's values, where x alone is less than `want`
-  ClosureGrid(int64_t K, int values, int most, int64_t want) : per_block(most) {
+  dim3 grid;      // x: elements; y: parts of an element's values, where x alone is less than `parts`
+  ClosureGrid(int64_t K, int values, int most, int64_t want, int64_t parts) : per_block(most) {
     while (per_block > 1 && (K + per_block - 1) / per_block < want) per_block /= 2;
     threads = std::min(256, std::max(64, (values + 31) / 32 * 32));
     const int64_t x = (K + per_block - 1) / per_block;
     grid = dim3((unsigned)std::min<int64_t>(x, INT32_MAX),
-                (unsigned)std::min<int64_t>((values + threads - 1) / threads, (want + x - 1) / x));
+                (unsigned)std::min<int64_t>((values + threads - 1) / threads, (parts + x - 1) / x));
   }
 };
 
@@ -550,7 +554,8 @@ extern "C" int bb_closure_features(bb_ctx* ctx, int N, int64_t K, int nf, const 
   int* status = bb_ctx_status_word(ctx);
   if (!status) return bb_fail(ctx, BB_ERR_NOMEM, "status word allocation failed");
   cudaStream_t st = (cudaStream_t)stream;
-  const ClosureGrid g(K, nf * (np3(N) + 4 * np2(N)), kFeatureElems, 4 * ctx->num_sms);
+  const int64_t want = 4 * ctx->num_sms;
+  const ClosureGrid g(K, nf * (np3(N) + 4 * np2(N)), kFeatureElems, want, want);
   const int per_block = g.per_block;
   auto go = [&](auto kern, auto* qt) {
     kern<<<g.grid, g.threads, 0, st>>>(t->d_words, t->o_fvol, t->o_fperm, N, K, nf, conn, qt, scale,
@@ -581,7 +586,8 @@ extern "C" int bb_closure_apply(bb_ctx* ctx, int N, int64_t K, int nf, int dtype
   if (K == 0) return BB_OK;
   cudaStream_t st = (cudaStream_t)stream;
   // in double the conversions bound few elements, so they are spread wider
-  const ClosureGrid g(K, nf * np3(N), kApplyElems, (dtype == BB_F64 ? 4 : 1) * ctx->num_sms);
+  const ClosureGrid g(K, nf * np3(N), kApplyElems, (dtype == BB_F64 ? 4 : 1) * ctx->num_sms,
+                      16 * ctx->num_sms);
   const int per_block = g.per_block;
   if (K / per_block >= INT32_MAX) return bb_fail(ctx, BB_ERR_ARG, "bad argument to bb_closure_apply");
   auto go = [&](auto kern, auto* qt) {
