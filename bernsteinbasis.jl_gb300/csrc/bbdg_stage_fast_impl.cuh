@@ -371,14 +371,22 @@ __device__ __forceinline__ void lift_pair_warp(const float* xa, const float* xb,
   }
 }
 
+// Kernels that form the penalty weights with a square root and a division instead of face_weights: the
+// degrees from generic_order on, for the generic kernel's very bits, and Maxwell N = 10, which the steps
+// slow down more where there are many tiles (two time steps with the bare approximation / that pair /
+// the steps: K = 16,464, 2,366 / 2,381 / 2,442 us; K = 3,072, 484 / 493 / 486).
+template <int PHYS>
+__host__ __device__ constexpr bool library_weights(int N) {
+  return generic_order(N) || (PHYS == BB_MAXWELL && N == 10);
+}
+
 // The penalty weights cp = tau |n| and cu = tau / |n| from n2 = |n|^2. The approximate reciprocal
 // root (2 ulp) gets one Newton step for the root and one for the quotient, their remainders in
 // fused operations (Markstein, Computation of elementary functions on the IBM RISC System/6000
 // processor, 1990), which makes them as accurate as a square root and a division rounded to the
 // nearest. The library's pair costs 1 to 4 % of a stage (Maxwell N = 5, K = 48,000, four steps: 2,446
 // us with the bare approximation, 2,545 with the pair, 2,455 with the steps; wave N = 9, K = 196,608,
-// one step: 4,584 / 4,609 / 4,593; Maxwell N = 10, K = 16,464, four steps: 4,683 / 4,700 / 4,823).
-// Degrees from generic_order on take that pair all the same, for the generic kernel's very bits.
+// one step: 4,584 / 4,609 / 4,593).
 __device__ __forceinline__ void face_weights(float n2, float tau, float& cp, float& cu) {
   const float r = rsqrtf(n2), l0 = n2 * r, u0 = tau * r;
   const float l = fmaf(fmaf(-l0, l0, n2), 0.5f * r, l0);
@@ -570,7 +578,7 @@ __global__ void __launch_bounds__(FastLayout<N, PHYS, EPB, TPE>::NT,
     float cp = 1.f, cu = 1.f;
     if (tau > 0.f) {
       const float n2 = nx * nx + ny * ny + nz * nz;
-      if constexpr (generic_order(N)) {
+      if constexpr (library_weights<PHYS>(N)) {
         const float Jf = sqrtf(n2);
         cp = tau * Jf;
         cu = tau / Jf;
