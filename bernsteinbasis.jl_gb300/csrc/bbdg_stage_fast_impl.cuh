@@ -4,8 +4,8 @@
 //
 // Same algorithm and data layout as the generic stage kernel (bbdg_solver.cu) with the
 // degree N a compile-time constant, which turns every multi-index computation into an
-// immediate and lets one thread run a whole face lift chain in registers (high degrees: a pair
-// of warps works level by level on a face, lift_pair_warp):
+// immediate and lets one thread run a whole face lift chain in registers (high degrees: a warp
+// works level by level on a pair of a face's chains, lift_pair_warp):
 //
 //   lift, per face f and chain c (src/BernsteinLift.jl:139-164):
 //     E0 = L0 x,  L0 = (N+1)^2/2 R_{N+1} E_{N->N+1}, applied as its 7-point stencil
